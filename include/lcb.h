@@ -139,7 +139,8 @@ int lcb_plasma_move_deposit(const lcb_move_deposit_args *a, void *stream);
  * and of the DCT-I matrix c_j cos(pi j k/(N-1)) (order N), and the
  * reference's Dirichlet, mixed (and its transpose) and Neumann solver
  * matrices (lcode/plasma3d/initialization.py:15-67), in FP64, or in FP32
- * for LCB_PREC_MIXED.  subtraction_coeff is the Helmholtz shift of the mixed
+ * for LCB_PREC_MIXED, and behind them the FP64 tables of the fast transforms
+ * where the grid has them.  subtraction_coeff is the Helmholtz shift of the mixed
  * matrix ('field-solver-subtraction-coefficient' after the 3D adjustment). */
 size_t lcb_field_operators_bytes(int grid_steps, int precision);
 int lcb_field_operators_build(int grid_steps, double h, double subtraction_coeff,
@@ -184,12 +185,14 @@ typedef struct lcb_compute_fields_args {
  * (device, grid_steps, precision) that is not under stream capture times
  * both on the caller's stream and keeps the faster (it computes the same
  * outputs several times and synchronises the stream once).
- * LCB_WAVE_KERNEL=tiled or =persistent in the environment fixes the choice. */
+ * LCB_WAVE_KERNEL=tiled or =persistent in the environment fixes the choice,
+ * for every grid. */
 int lcb_compute_fields(const lcb_compute_fields_args *a, void *stream);
 size_t lcb_compute_fields_workspace_bytes(int grid_steps, int precision);
 
 /* The wave kernel chosen for (grid_steps, precision) on the current device:
- * 1 one CTA per tile, 2 persistent, 0 not measured yet.  No counterpart in
+ * 1 one CTA per tile, 2 persistent, 0 not measured yet, 3 none (the grid is
+ * solved by fast transforms).  No counterpart in
  * the reference (reporting only). */
 int lcb_wave_kernel_choice(int grid_steps, int precision);
 

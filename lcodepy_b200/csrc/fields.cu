@@ -1,6 +1,8 @@
-// Field solver: right-hand sides, then every DST-I / DCT-I / mixed transform
-// pair of compute_fields (lcode/plasma3d/fields.py:176-322) as four waves of
-// one batched dense matrix product each, then the finishing epilogues.
+// Field solver by dense products, for grids that have no fast transforms
+// (spectral.cu), and the entry points of both: right-hand sides, then every
+// DST-I / DCT-I / mixed transform pair of compute_fields
+// (lcode/plasma3d/fields.py:176-322) as four waves of one batched dense
+// matrix product each, then the finishing epilogues.
 //
 // Seven problems per call, in this order (n = N - 2):
 //   0 Ey, 1 Bx : X = rhs[1:-1, :]   (n x N); out = S (M  o (S X C^T)) C^T
@@ -32,6 +34,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "spectral.cuh"
 
 namespace lcb {
 
@@ -1762,11 +1765,40 @@ static int solve(const lcb_compute_fields_args *a, const T *ops, cudaStream_t st
 
 using namespace lcb;
 
+namespace lcb {
+
+// LCB_WAVE_KERNEL: 0 unset, else the wave kernel fixed for every grid.
+static int wave_kernel_env()
+{
+    static const int mode = [] {
+        const char *v = getenv("LCB_WAVE_KERNEL");
+        if (v && strcmp(v, "tiled") == 0) return (int)WK_TILED;
+        if (v && strcmp(v, "persistent") == 0) return (int)WK_PERSISTENT;
+        return 0;
+    }();
+    return mode;
+}
+
+// Grids solved by fast transforms (spectral.cu): all whose N - 1 factors into
+// primes up to 13, unless LCB_WAVE_KERNEL asks for the dense products.
+static bool by_fast_transforms(int N) { return !wave_kernel_env() && spectral_grid(N); }
+
+// The operator buffer: the dense operators, then for grids with fast
+// transforms their tables, from the next multiple of 256 bytes on.
+static size_t dense_ops_bytes(int N, int precision)
+{
+    const size_t el = precision == LCB_PREC_MIXED ? sizeof(float) : sizeof(double);
+    return ((size_t)op_layout(N).off[OP_COUNT] * el + 255) / 256 * 256;
+}
+
+}  // namespace lcb
+
 extern "C" size_t lcb_field_operators_bytes(int grid_steps, int precision)
 {
     if (grid_steps < 5 || (grid_steps % 2) == 0) return 0;
     const size_t el = precision == LCB_PREC_MIXED ? sizeof(float) : sizeof(double);
-    return (size_t)op_layout(grid_steps).off[OP_COUNT] * el;
+    if (!spectral_grid(grid_steps)) return (size_t)op_layout(grid_steps).off[OP_COUNT] * el;
+    return dense_ops_bytes(grid_steps, precision) + spectral_ops_bytes(grid_steps);
 }
 
 extern "C" int lcb_field_operators_build(int grid_steps, double h, double subtraction_coeff,
@@ -1798,6 +1830,10 @@ extern "C" int lcb_field_operators_build(int grid_steps, double h, double subtra
         k_build_slices<8><<<sblocks, 256, 0, as_stream(stream)>>>(N, L, static_cast<uint8_t *>(operators));
     }
     LCB_LAUNCH_CHECK("k_build_slices");
+    if (spectral_grid(N))
+        return spectral_ops_build(N, h, subtraction_coeff,
+                                  static_cast<char *>(operators) + dense_ops_bytes(N, precision),
+                                  as_stream(stream));
     return LCB_OK;
 }
 
@@ -1827,17 +1863,6 @@ namespace lcb {
 
 static std::mutex g_tune_mu;
 static std::map<std::tuple<int, int, int>, int> g_tuned;   // (device, N, precision) -> WK_*
-
-static int wave_kernel_env()
-{
-    static const int mode = [] {
-        const char *v = getenv("LCB_WAVE_KERNEL");
-        if (v && strcmp(v, "tiled") == 0) return (int)WK_TILED;
-        if (v && strcmp(v, "persistent") == 0) return (int)WK_PERSISTENT;
-        return 0;
-    }();
-    return mode;
-}
 
 template <typename T>
 static int solve_tuned(const lcb_compute_fields_args *a, const T *ops, cudaStream_t st)
@@ -1893,6 +1918,7 @@ static int solve_tuned(const lcb_compute_fields_args *a, const T *ops, cudaStrea
 
 extern "C" int lcb_wave_kernel_choice(int grid_steps, int precision)
 {
+    if (by_fast_transforms(grid_steps)) return 3;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     std::lock_guard<std::mutex> lock(lcb::g_tune_mu);
@@ -1917,10 +1943,12 @@ extern "C" int lcb_compute_fields(const lcb_compute_fields_args *a, void *stream
     LCB_REQUIRE(a->rho_beam_divisor != 0.0, "rho_beam_divisor is 0");
     for (int f : {0, 1, 3, 4}) LCB_REQUIRE(a->fields.f[f], "fields plane %d is NULL", f);
     for (int f = 0; f < 6; f++) LCB_REQUIRE(a->fields_prev.f[f], "fields_prev plane %d is NULL", f);
+    LCB_REQUIRE(a->precision == LCB_PREC_FP64 || a->precision == LCB_PREC_MIXED, "bad precision %d", a->precision);
     cudaStream_t st = as_stream(stream);
+    if (by_fast_transforms(N))
+        return spectral_solve(a, static_cast<const char *>(a->operators) + dense_ops_bytes(N, a->precision), st);
     if (a->precision == LCB_PREC_MIXED)
         return solve_tuned<float>(a, static_cast<const float *>(a->operators), st);
-    LCB_REQUIRE(a->precision == LCB_PREC_FP64, "bad precision %d", a->precision);
     return solve_tuned<double>(a, static_cast<const double *>(a->operators), st);
 }
 
