@@ -396,18 +396,30 @@ static size_t deposit_smem_bytes()
 // Fused predictor-corrector stage: K2 (move_smart) followed by K3 (deposit)
 // of the same particles, and for the first stage of an xi step K1 (the
 // free-streaming estimate) in front (move.py:169-313, weights.py:151-190).
-// A block owns a lattice tile of TI x TJ particles; the six field planes are
-// staged in a shared-memory window around the tile for the midpoint gather,
-// and the new position is deposited into a second window, flushed with
-// global atomics; particles whose stencil leaves a window use global memory.
-// FP64 (FT = double): each particle's gather and push are those of K2 and
-// K3 (same quotients, same summation order); the deposit sums the two
-// particles of a cell before the shared atomic.  Mixed precision
+// A block owns a lattice tile of TI x TJ particles.  The six field planes are
+// staged in a shared-memory window around the tile for the midpoint gather;
+// the moved particles are then sorted by cell (counts, a scan, records of
+// their weights and values in shared memory), and their stencils summed in
+// registers, a lane taking four cells along x and one quantity, before the
+// sums go to HBM: about 16 additions per particle instead of 100 in shared
+// memory.  Particles whose stencil leaves a window use global memory.
+// FP64 (FT = double): FP64 window, weights and sums.  Mixed precision
 // (FT = float): coordinates and momenta stay FP64; the gather reads an FP32
-// copy of the field window with FP32 weights (the planes come from the FP32
-// field solve); the deposit keeps FP64 weights, scales each particle's four
-// values by 2^32 / h^2 once, and rounds every contribution to a 64-bit
-// integer with one FMA against FIX_MAGIC, summed with integer atomics.
+// copy of the field window with FP32 weights (the mixed form's fields carry
+// FP32 accuracy); the deposit keeps FP64 weights, scales each particle's four
+// values by 2^32 / h^2 once, and rounds every contribution to an integer with
+// one FMA against FIX_MAGIC, so that the sums are exact.
+//
+// What bounds it: latency, at the 16 warps per SM that the push's registers
+// leave.  Adding every contribution to a shared window with 32-bit integer
+// atomics (three words a sum in FP64, two in mixed precision) kept the
+// shared-memory pipe 75 % busy and took 145 / 112 us for 929,296 particles
+// behind a driver (FP64 / mixed, with the clearing of the planes); this form
+// takes 101 / 94 us (with the background's copy folded into the clearing; 107
+// before that).  Also measured, at 107 / 94: the contraction on the FP64 matrix
+// instructions (121 / 114 us; m8n8k4 runs at a third of the vector rate for
+// this shape), columns of cells walked with a sliding sum (119 / 107 us), and
+// a deposit kernel of its own (121 / 125 us).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void weights4f(float x, float w[5])
 {
@@ -531,152 +543,96 @@ __device__ __forceinline__ void gather_one(const unsigned char *sf, const double
     }
 }
 
-// The shared-memory window keeps each fixed-point sum as two 32-bit words,
-// because 32-bit integer atomics are native in shared memory and 64-bit ones
-// are not: a contribution c (in units of 2^-32) adds its low 20 bits to an
-// unsigned word and c >> 20 to a signed word; the flush recombines
-// (hi << 20) + lo exactly.  A block adds at most 2 x 256 contributions to a
-// cell, so the low word stays below 2^29 and, with |c| < 2^41 (particles
-// whose scaled values reach 2^42, i.e. |value| / h^2 >= 1024, take the
-// global 64-bit path instead), the high word below 2^30.
-constexpr double FIX_SHARED_LIMIT = 4398046511104.0;   // 2^42, on values scaled by 2^32 / h^2
+// Values (in units of 2^-32, with the 1/h^2 of the weights) whose sums over
+// a block's particles stay far inside the integers that fit FIX_MAGIC's
+// binade (512 x 2^42 x 0.36 < 2^51); larger ones go straight to HBM.
+constexpr double FIX_SHARED_LIMIT = 4398046511104.0;   // 2^42
 
-// t = FIX_MAGIC + c exactly (the rounding FMA's result).  FIX_MAGIC's low
-// word is zero, so the low word of t's bit pattern is c mod 2^32 and its high
-// word minus 0x43380000 is floor(c / 2^32); c >> 20 is then one funnel shift.
-__device__ __forceinline__ void shared_fix_add(unsigned *lo, int *hi, int idx, double t)
+__device__ __forceinline__ double max_abs4(const double (&v)[4])
 {
-    const unsigned w0 = (unsigned)__double2loint(t);
-    const unsigned w1 = (unsigned)(__double2hiint(t) - 0x43380000);
-    atomicAdd(lo + idx, w0 & 0xFFFFFu);
-    atomicAdd(hi + idx, (int)__funnelshift_r(w0, w1, 20));
+    return fmax(fmax(fabs(v[0]), fabs(v[1])), fmax(fabs(v[2]), fabs(v[3])));
 }
 
-__device__ __forceinline__ bool shared_fix_ok(const double sv[4])
+// One particle's deposit into HBM (weights.py:151-190 arithmetic): its
+// stencil leaves the window, or its values the range that a block sums (FP64:
+// infinities and NaN); sv: its values with the 1/h^2 (mixed: in fixed-point
+// units).
+template <typename FT, typename Acc>
+__device__ __forceinline__ void deposit_direct(Acc *const (&g)[4], int N, int cx, int cy, double xl,
+                                               double yl, const double (&sv)[4])
 {
-    return fmax(fmax(fabs(sv[0]), fabs(sv[1])), fmax(fabs(sv[2]), fabs(sv[3]))) < FIX_SHARED_LIMIT;
-}
-
-// Deposit of one particle's scaled values (FP64 weights, fixed-point sums).
-template <int WX, int WY>
-__device__ __forceinline__ void deposit_fix_one(unsigned *swl, int *swh, fix_t *const *g, int N,
-                                                int wx0, int wy0, int cx, int cy, double xl,
-                                                double yl, const double sv[4])
-{
-    constexpr int WSZ = WX * WY;
     double wx[5], wy[5];
     weights4(xl, wx);
     weights4(yl, wy);
-    const int lx = cx - 2 - wx0, ly = cy - 2 - wy0;
-    if (lx >= 0 && lx + 5 <= WX && ly >= 0 && ly + 5 <= WY && shared_fix_ok(sv)) {
-#pragma unroll
-        for (int a = 0; a < 5; a++) {
-#pragma unroll
-            for (int b = 0; b < 5; b++) {
-                const double w = wx[a] * wy[b];
-                const int c = (lx + a) * WY + ly + b;
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    shared_fix_add(swl, swh, q * WSZ + c, fma(sv[q], w, FIX_MAGIC));
-            }
-        }
-    } else {
+    int64_t row = (int64_t)(cx - 2) * N + cy - 2;
 #pragma unroll 1
-        for (int a = 0; a < 5; a++) {
-#pragma unroll
-            for (int b = 0; b < 5; b++) {
-                const double w = wx[a] * wy[b];
-                const int64_t c = (int64_t)(cx + a - 2) * N + cy + b - 2;
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    atomicAdd(g[q] + c, fix_bits(fma(sv[q], w, FIX_MAGIC)));
-            }
-        }
-    }
-}
-
-// FP64 deposit window: every contribution v (an FP64 value in the units of
-// the output currents) is rounded to a multiple of 2^-56 and summed as an
-// integer split over three 32-bit words -- bits 0-19 and 20-39 unsigned,
-// bits 40 up signed -- with 32-bit shared integer atomics, which run the
-// fused stage about 7% faster than FP64 shared atomics.  A particle whose
-// contributions could reach |v| = 2^4 (weights wx wy are below 0.36)
-// deposits into HBM with FP64 atomics instead, so |v| 2^56 <
-// 2^60 and, with at most 2 x 256 contributions per cell and block (every
-// particle of the block at most once), no word overflows.  The integer sums
-// are exact and independent of the order of the atomics; each contribution
-// differs from FP64 by at most 2^-57, and the flush recombines the words
-// with one FP64 rounding before adding the value to the outputs.  The
-// particle's values arrive multiplied by 2^56 (exact: a power of two), so a
-// contribution's integer is one rounding conversion of its product.
-constexpr double FIX56_SCALE = 72057594037927936.0;   // 2^56
-constexpr double FIX56_LIMIT = 16.0 * FIX56_SCALE;    // per contribution, in the window
-
-// v: a contribution in units of 2^-56
-__device__ __forceinline__ void fix56_add(unsigned *w0, unsigned *w1, int *w2, int idx, double v)
-{
-    const long long c = __double2ll_rn(v);
-    atomicAdd(w0 + idx, (unsigned)c & 0xFFFFFu);
-    atomicAdd(w1 + idx, (unsigned)(c >> 20) & 0xFFFFFu);
-    atomicAdd(w2 + idx, (int)(c >> 40));
-}
-
-__device__ __forceinline__ double fix56_value(unsigned w0, unsigned w1, int w2)
-{
-    return ((double)w2 * 1099511627776.0 + (double)w1 * 1048576.0 + (double)w0) * (1.0 / FIX56_SCALE);
-}
-
-// One particle's FP64 deposit (weights.py:151-190 arithmetic, w = (wx / h)
-// (wy / h)) into the three-word window, or into HBM with FP64 atomics when
-// the stencil leaves the window or a contribution could leave the range;
-// sv: the particle's values in units of 2^-56.
-template <int WX, int WY>
-__device__ __forceinline__ void deposit_fix56_one(unsigned *w0, unsigned *w1, int *w2, double *const *g,
-                                                  int N, double ih, int wx0, int wy0, int cx, int cy,
-                                                  double xl, double yl, const double sv[4])
-{
-    constexpr int WSZ = WX * WY;
-    double wx[5], wy[5];
-    weights4(xl, wx);
-    weights4(yl, wy);
-#pragma unroll
-    for (int b = 0; b < 5; b++) wy[b] *= ih;
-    const int lx = cx - 2 - wx0, ly = cy - 2 - wy0;
-    const double m = fmax(fmax(fabs(sv[0]), fabs(sv[1])), fmax(fabs(sv[2]), fabs(sv[3])));
-    const bool inwin = lx >= 0 && lx + 5 <= WX && ly >= 0 && ly + 5 <= WY &&
-                       m * (0.36 * ih * ih) < FIX56_LIMIT;
-#pragma unroll
     for (int a = 0; a < 5; a++) {
-        const double wxa = wx[a] * ih;
 #pragma unroll
         for (int b = 0; b < 5; b++) {
-            const double w = wxa * wy[b];
-            if (inwin) {
-                const int c = (lx + a) * WY + ly + b;
+            const double w = wx[0] * wy[b];
 #pragma unroll
-                for (int q = 0; q < 4; q++) fix56_add(w0, w1, w2, q * WSZ + c, sv[q] * w);
-            } else {
-                const int64_t c = (int64_t)(cx + a - 2) * N + cy + b - 2;
-#pragma unroll
-                for (int q = 0; q < 4; q++) atomicAdd(g[q] + c, sv[q] * w * (1.0 / FIX56_SCALE));
+            for (int q = 0; q < 4; q++) {
+                if constexpr (sizeof(FT) == 4) atomicAdd(g[q] + row + b, fix_bits(fma(sv[q], w, FIX_MAGIC)));
+                else atomicAdd(g[q] + row + b, sv[q] * w);
             }
         }
+#pragma unroll
+        for (int k = 0; k < 4; k++) wx[k] = wx[k + 1];
+        row += N;
     }
 }
 
-// A thread owns two particles, lattice slots t and t + DEP_THREADS, which on
-// the 2 x 2 per cell lattice are the two lattice rows of one cell.  While
-// both sit in the same cell the window values of the gather are loaded once
-// for the two, and their deposits are added before the shared atomics (each
-// contribution is still rounded on its own: fma(sA, wA, fma(sB, wB, M)) adds
-// two integers), which halves the shared-memory traffic of both phases.
 template <typename FT> struct StageAcc;
 template <> struct StageAcc<float> { typedef fix_t type; };
 template <> struct StageAcc<double> { typedef double type; };
 
-template <typename FT, int WX, int WY, bool FIRST>
-__global__ void __launch_bounds__(DEP_THREADS, sizeof(FT) == 4 ? 3 : 2)
-k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step, double boundary,
+// 1 / x and sqrt(x) for normal positive x by Newton's method from the
+// hardware's approximations (about 2^-20): a step of third order for the
+// reciprocal, two coupled second-order steps for the root, within two units
+// in the last place.  Shorter chains than the correctly rounded operations;
+// a stage has four to five of each per particle in sequence.
+__device__ __forceinline__ double rcp_nr(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double sqrt_nr(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    const double e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    return fma(fma(-g, g, x), h, g);
+}
+
+// Shape of a block of the fused stage: TI x TJ lattice particles, two per
+// thread; a window of WX x WY nodes around them.
+template <typename FT, int WX_, int WY_> struct Stage {
+    static constexpr int TI = 16, TJ = 32, WX = WX_, WY = WY_;
+    static constexpr int NP = TI * TJ, THREADS = NP / 2, WARPS = THREADS / 32;
+    static constexpr int WSZ = WX * WY;
+    static constexpr int CX = WX - 4, CY = WY - 4, NC = CX * CY;   // cells of the window
+    // cells along x that one lane of the deposit sums (4: 107 us a production
+    // FP64 stage, 3: 109, 5: 111; with another record layout 4: 114, 1: 129)
+    static constexpr int XU = 4;
+    // a particle's record for the deposit: five weights along x, five along
+    // y, four values; the cells' columns a record apart (neighbouring lanes
+    // write to and read from neighbouring columns, some 40 records away, and
+    // shall not meet in a bank)
+    static constexpr int RECORD = 14, SLOTS = NP + CY;
+    static constexpr size_t field_bytes = (size_t)WSZ * FieldWin<FT>::bytes_per_cell;
+    static constexpr size_t rec_bytes = (size_t)SLOTS * RECORD * sizeof(double);
+    static constexpr size_t main_bytes = field_bytes > rec_bytes ? field_bytes : rec_bytes;
+    static constexpr size_t smem = main_bytes + (NC + 1 + WARPS + 4) * sizeof(int);
+};
+
+template <typename S, typename FT, bool FIRST>
+__global__ void __launch_bounds__(S::THREADS, 2)
+k_move_deposit(int64_t n_per_sort, int Ns, int N, int fineness, double h, double xi_step, double boundary,
                   const double *__restrict__ Exf, const double *__restrict__ Eyf,
                   const double *__restrict__ Ezf, const double *__restrict__ Bxf,
                   const double *__restrict__ Byf, const double *__restrict__ Bzf,
@@ -695,17 +651,15 @@ k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step,
     pdl_trigger();
     constexpr bool MIXED = sizeof(FT) == 4;
     typedef typename StageAcc<FT>::type Acc;
-    static_assert(DEP_PPT == 2, "a thread owns two particles");
-    constexpr int WSZ = WX * WY;
+    constexpr int WX = S::WX, WY = S::WY, WSZ = S::WSZ, THREADS = S::THREADS;
+    constexpr int CX = S::CX, NC = S::NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // deposit window: mixed, [4][WX][WY] low and high words of the 2^-32
-    // fixed-point sums; FP64, three words per sum of the 2^-56 ones
-    constexpr int DEP_WORDS = MIXED ? 2 : 3;
-    unsigned *swl = reinterpret_cast<unsigned *>(smem_raw);    // [4][WX][WY] word 0
-    int *swh = reinterpret_cast<int *>(swl + 4 * WSZ);         // mixed: high words
-    unsigned *sw1 = swl + 4 * WSZ;                             // FP64: words 1 and 2
-    int *sw2 = reinterpret_cast<int *>(swl + 8 * WSZ);
-    unsigned char *sf = smem_raw + (size_t)DEP_WORDS * 4 * WSZ * 4;  // fields, FieldWin
+    // the field window (FieldWin); after the gather, over it, the particles'
+    // records in the order of their cells
+    unsigned char *sf = smem_raw;
+    double *rec = reinterpret_cast<double *>(smem_raw);
+    int *start = reinterpret_cast<int *>(smem_raw + S::main_bytes);   // [NC + 1] first records
+    int *wsum = start + NC + 1, *box = wsum + S::WARPS;
     const int s = blockIdx.z;
     const int64_t base = (int64_t)s * n_per_sort;
     const int half_n = N / 2;
@@ -714,84 +668,86 @@ k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step,
     const double *const fld[6] = {Exf, Eyf, Ezf, Bxf, Byf, Bzf};
     const double ih = 1.0 / h;
 
-    // Tiles start on a lattice row whose cell also holds the next row, so
-    // that a thread's two rows (ti, ti + 1 with ti even) share a cell: when
-    // rows 0 and 1 sit in different cells the tiles are shifted up by one
-    // row (the grid has one spare row of tiles for it).  The tile's first
-    // particle is read for both possible shifts at once, so that the tile
-    // origin costs one round trip to memory.
-    double dummy;
-    const int ia = blockIdx.y * DEP_TI, ib = ia > 0 ? ia - 1 : 0;   // tile row for off = 0, 1
-    const int64_t ka = base + (int64_t)(ia < Ns ? ia : 0) * Ns + blockIdx.x * DEP_TJ;
-    const int64_t kb = base + (int64_t)ib * Ns + blockIdx.x * DEP_TJ;
-    const bool two_rows = Ns > 1;
-    const double r0x = x_init[base], r1x = two_rows ? x_init[base + Ns] : r0x;
-    const double xa = x_init[ka], ya = y_init[ka], xb = x_init[kb], yb = y_init[kb];
-    const double xa1 = ia + 1 < Ns ? x_init[ka + Ns] : xa, xb1 = ib + 1 < Ns ? x_init[kb + Ns] : xb;
-    const int off = (two_rows && cell_of(r0x / h + 0.5, half_n, dummy) !=
-                                 cell_of(r1x / h + 0.5, half_n, dummy)) ? 1 : 0;
-    const int i0 = blockIdx.y * DEP_TI - off, j0 = blockIdx.x * DEP_TJ;
-    const int ir = i0 < 0 ? 0 : i0;
-    if (ir >= Ns) return;
-    const int64_t k0 = base + (int64_t)ir * Ns + j0;
-    const double x0 = off ? xb : xa, y0 = off ? yb : ya, x1 = off ? xb1 : xa1;
-    const int wx0 = cell_of(x0 / h + 0.5, half_n, dummy) - 2 - DEP_SLACK;
-    const int wy0 = cell_of(y0 / h + 0.5, half_n, dummy) - 2 - DEP_SLACK;
-    bool two = false;
-    if (ir + 1 < Ns) {
-        const double d = x1 - x0;
-        two = fabs(2 * d - h) < 0.25 * h;
-    }
-    (void)k0;
-
-    // ---- the particles' first loads, issued before the window fill ----
+    // Lanes take consecutive particles of a lattice row (coalesced loads;
+    // neighbours in one cell read the same window values), a thread the rows
+    // i and i + 1.  Tiles start on a lattice row whose cell also holds the
+    // next row, so that a thread's two rows share a cell: when rows 0 and 1
+    // sit in different cells the tiles are shifted up by one row (the grid has
+    // one spare row of tiles for it).  The loads are issued for what the
+    // package's own lattice needs (a shift with two particles per cell) before
+    // the lattice is looked at, and again if it is another one.
+    const int row = 2 * (threadIdx.x / S::TJ), j = blockIdx.x * S::TJ + threadIdx.x % S::TJ;
     int64_t kk[2];
     bool live[2], zero_p[2];
     double L_xo0[2], L_yo0[2], L_xi[2], L_yi[2], L_q[2], L_xof[2], L_yof[2];
-    double L_m[2], L_px[2], L_py[2], L_pz[2];
+    double L_m[2], L_px[2], L_py[2], L_pz[2], x0, y0;
+    auto load = [&](int off) {
+        const int i0 = blockIdx.y * S::TI - off;
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
-        int ti, tj;
-        tile_slot(threadIdx.x + p * DEP_THREADS, two, ti, tj);
-        const int i = i0 + ti, j = j0 + tj;
-        live[p] = i >= 0 && i < Ns && j < Ns;
-        kk[p] = base + (int64_t)i * Ns + j;
-        L_xo0[p] = L_yo0[p] = L_xi[p] = L_yi[p] = L_q[p] = L_xof[p] = L_yof[p] = 0;
-        L_m[p] = L_px[p] = L_py[p] = L_pz[p] = 0;
-        if (!live[p]) continue;
-        const int64_t k = kk[p];
-        L_xo0[p] = xo_p[k]; L_yo0[p] = yo_p[k];
-        L_xi[p] = x_init[k]; L_yi[p] = y_init[k];
-        if (FIRST) {
-            L_m[p] = m_a[k]; L_px[p] = px_p[k]; L_py[p] = py_p[k]; L_pz[p] = pz_p[k];
-            L_q[p] = q_p[k];
-        } else {
-            L_q[p] = q_f[k]; L_xof[p] = xo_f[k]; L_yof[p] = yo_f[k];
+        for (int p = 0; p < 2; p++) {
+            const int i = i0 + row + p;
+            live[p] = i >= 0 && i < Ns && j < Ns;
+            const int64_t k = kk[p] = base + (int64_t)i * Ns + j;
+            L_xo0[p] = L_yo0[p] = L_xi[p] = L_yi[p] = L_q[p] = L_xof[p] = L_yof[p] = 0;
+            L_m[p] = L_px[p] = L_py[p] = L_pz[p] = 0;
+            if (!live[p]) continue;
+            L_xo0[p] = xo_p[k]; L_yo0[p] = yo_p[k];
+            L_xi[p] = x_init[k]; L_yi[p] = y_init[k];
+            if (FIRST) {
+                L_m[p] = m_a[k]; L_px[p] = px_p[k]; L_py[p] = py_p[k]; L_pz[p] = pz_p[k];
+                L_q[p] = q_p[k];
+            } else {
+                L_q[p] = q_f[k]; L_xof[p] = xo_f[k]; L_yof[p] = yo_f[k];
+            }
         }
-    }
-
-    for (int t = threadIdx.x; t < DEP_WORDS * 4 * WSZ; t += blockDim.x) swl[t] = 0u;
+        // the tile's first particle
+        const int ir = i0 < 0 ? 0 : i0;
+        const int64_t k0 = base + (int64_t)(ir < Ns ? ir : 0) * Ns + blockIdx.x * S::TJ;
+        x0 = x_init[k0]; y0 = y_init[k0];
+    };
     // the field window, FILL_BATCH cells per thread at a time: the batch's
     // loads are all in flight before the first store to the window
-    constexpr int FILL_ITERS = (WSZ + DEP_THREADS - 1) / DEP_THREADS, FILL_BATCH = 3;
+    auto fill = [&](int wx0, int wy0) {
+        constexpr int FILL_ITERS = (WSZ + THREADS - 1) / THREADS, FILL_BATCH = 3;
 #pragma unroll
-    for (int k0 = 0; k0 < FILL_ITERS; k0 += FILL_BATCH) {
-        FT v[FILL_BATCH][6];
+        for (int k0 = 0; k0 < FILL_ITERS; k0 += FILL_BATCH) {
+            FT v[FILL_BATCH][6];
 #pragma unroll
-        for (int k = 0; k < FILL_BATCH; k++) {
-            const int t = threadIdx.x + (k0 + k) * DEP_THREADS;
-            const int gx = wx0 + t / WY, gy = wy0 + t % WY;
-            const bool in = k0 + k < FILL_ITERS && t < WSZ && gx >= 0 && gx < N && gy >= 0 && gy < N;
-            const int64_t g = (int64_t)gx * N + gy;
+            for (int k = 0; k < FILL_BATCH; k++) {
+                const int t = threadIdx.x + (k0 + k) * THREADS;
+                const int gx = wx0 + t / WY, gy = wy0 + t % WY;
+                const bool in = k0 + k < FILL_ITERS && t < WSZ && gx >= 0 && gx < N && gy >= 0 && gy < N;
+                const int64_t g = (int64_t)gx * N + gy;
 #pragma unroll
-            for (int f = 0; f < 6; f++) v[k][f] = in ? (FT)__ldg(fld[f] + g) : FT(0);
+                for (int f = 0; f < 6; f++) v[k][f] = in ? (FT)__ldg(fld[f] + g) : FT(0);
+            }
+#pragma unroll
+            for (int k = 0; k < FILL_BATCH; k++) {
+                const int t = threadIdx.x + (k0 + k) * THREADS;
+                if (k0 + k < FILL_ITERS && t < WSZ) FieldWin<FT>::put(sf, WSZ, t, v[k]);
+            }
         }
-#pragma unroll
-        for (int k = 0; k < FILL_BATCH; k++) {
-            const int t = threadIdx.x + (k0 + k) * DEP_THREADS;
-            if (k0 + k < FILL_ITERS && t < WSZ) FieldWin<FT>::put(sf, WSZ, t, v[k]);
-        }
-    }
+    };
+    // The window around the tile's first particle: where a lattice centred on
+    // the grid with `fineness` particles per cell has it, so that the fields
+    // are asked for together with the particles, and where it is, if that is
+    // elsewhere.
+    double dummy;
+    auto origin = [&](double x) { return cell_of(x * ih + 0.5, half_n, dummy) - 2 - DEP_SLACK; };
+    const double lat = h / fineness, mid = 0.5 * (Ns - 1);
+    const int shift = fineness == 2;
+    const double r0x = x_init[base], r1x = Ns > 1 ? x_init[base + Ns] : r0x;
+    load(shift);
+    const int px = origin((max((int)blockIdx.y * S::TI - shift, 0) - mid) * lat);
+    const int py = origin(((int)blockIdx.x * S::TJ - mid) * lat);
+    fill(px, py);
+    for (int t = threadIdx.x; t <= NC; t += blockDim.x) start[t] = 0;
+    if (threadIdx.x < 4) box[threadIdx.x] = (threadIdx.x & 1) ? -1 : 0x7fffffff;
+    const int off = cell_of(r0x * ih + 0.5, half_n, dummy) != cell_of(r1x * ih + 0.5, half_n, dummy);
+    if (off != shift) load(off);
+    if ((int)blockIdx.y * S::TI - off >= Ns) return;
+    const int wx0 = origin(x0), wy0 = origin(y0);
+    if (wx0 != px || wy0 != py) fill(wx0, wy0);
     __syncthreads();
 
     // ---- phase 1: K1 (first stage) and the midpoint of each particle ----
@@ -811,8 +767,8 @@ k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step,
             const double mk = L_m[p], opx = L_px[p], opy = L_py[p], opz = L_pz[p];
             xof = xo0; yof = yo0;
             if (mk != 0) {
-                const double gm = sqrt(mk * mk + opz * opz + opx * opx + opy * opy);
-                const double adv = xi_step / (gm - opz);
+                const double gm = sqrt_nr(mk * mk + opz * opz + opx * opx + opy * opy);
+                const double adv = xi_step * rcp_nr(gm - opz);
                 xof += opx * adv;
                 yof += opy * adv;
             }
@@ -1003,18 +959,18 @@ k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step,
         double gm, dpx, dpy, dpz;
 #pragma unroll
         for (int it = 0; it < 2; it++) {
-            gm = sqrt(mk * mk + px * px + py * py + pz * pz);
+            gm = sqrt_nr(mk * mk + px * px + py * py + pz * pz);
             // f (E + v x B) with v = p / gm and f = q dxi / (1 - vz), as
             // q dxi (gm E + p x B) / (gm - pz): one quotient (algebraically
             // the reference's two, move.py:234-239)
-            const double r = qk * xi_step / (gm - pz);
+            const double r = qk * xi_step * rcp_nr(gm - pz);
             dpx = r * (gm * Ex + py * Bz - pz * By);
             dpy = r * (gm * Ey - px * Bz + pz * Bx);
             dpz = r * (gm * Ez + px * By - py * Bx);
             px = opx + dpx * 0.5; py = opy + dpy * 0.5; pz = opz + dpz * 0.5;
         }
-        gm = sqrt(mk * mk + px * px + py * py + pz * pz);
-        const double adv = xi_step / (gm - pz);
+        gm = sqrt_nr(mk * mk + px * px + py * py + pz * pz);
+        const double adv = xi_step * rcp_nr(gm - pz);
         double xo = xo_p[k] + px * adv;
         double yo = yo_p[k] + py * adv;
         px = opx + dpx; py = opy + dpy; pz = opz + dpz;
@@ -1032,10 +988,10 @@ k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step,
         px_f[k] = px; py_f[k] = py; pz_f[k] = pz;
         if (FIRST || absorbed) q_f[k] = absorbed ? 0.0 : qk;
         if (absorbed) continue;
-        const double gd = sqrt(mk * mk + px * px + py * py + pz * pz);
+        const double gd = sqrt_nr(mk * mk + px * px + py * py + pz * pz);
         // q / (1 - pz / gd) and p q / (gd - pz): one quotient (weights.py:
         // 164-168 has two)
-        const double r = qk / (gd - pz);
+        const double r = qk * rcp_nr(gd - pz);
         const double dro = r * gd, djx = r * px, djy = r * py, djz = r * pz;
         if (MIXED) check_range<fix_t>(dro, djx, djy, djz, ih, err);
         const int c_x = cell_of((xi0 + xo) * ih + 0.5, half_n, dxl[p]);
@@ -1045,188 +1001,161 @@ k_move_deposit_pair(int64_t n_per_sort, int Ns, int N, double h, double xi_step,
             continue;
         }
         cx[p] = c_x; cy[p] = c_y;
-        // values in fixed-point units: mixed, 2^32 (with the 1/h^2 of the
-        // weights); FP64, 2^56
-        const double sc = MIXED ? FIX_SCALE * ih * ih : FIX56_SCALE;
+        // with the 1/h^2 of the weights; mixed: in units of 2^-32
+        const double sc = (MIXED ? FIX_SCALE : 1.0) * ih * ih;
         sv[p][0] = dro * sc; sv[p][1] = djx * sc; sv[p][2] = djy * sc; sv[p][3] = djz * sc;
     }
 
     // ---- phase 4: deposit ----
-    // The gather's three forms again (warp-uniform choice), on the new cells.
-    const int mcx = min(cx[0], cx[1]), mcy = min(cy[0], cy[1]);
-    const int dx0 = mcx - 2 - wx0, dy0 = mcy - 2 - wy0;
-    const bool dpair = cx[0] >= 0 && cx[1] >= 0 && abs(cx[1] - cx[0]) <= 1 &&
-                       abs(cy[1] - cy[0]) <= 1 && dx0 >= 0 && dx0 + 6 <= WX && dy0 >= 0 &&
-                       dy0 + 6 <= WY;
-    const bool didle = cx[0] < 0 && cx[1] < 0;
-    if constexpr (MIXED) {
-        {
-            const int lx = cx[0] - 2 - wx0, ly = cy[0] - 2 - wy0;
-            const bool ok = shared_fix_ok(sv[0]) && shared_fix_ok(sv[1]);
-            const bool joint = cx[0] >= 0 && cx[0] == cx[1] && cy[0] == cy[1] &&
-                               lx >= 0 && lx + 5 <= WX && ly >= 0 && ly + 5 <= WY && ok;
-            if (!__all_sync(0xffffffffu, joint || didle)) {
-                if (dpair && ok) {
-                    double ax[6], ay[6], bx[6], by[6], t[5];
-                    weights4(dxl[0], t); shift6(t, cx[0] - mcx, ax);
-                    weights4(dyl[0], t); shift6(t, cy[0] - mcy, ay);
-                    weights4(dxl[1], t); shift6(t, cx[1] - mcx, bx);
-                    weights4(dyl[1], t); shift6(t, cy[1] - mcy, by);
-                    int row = dx0 * WY + dy0;
-#pragma unroll 1
-                    for (int a = 0; a < 6; a++) {
+    // Particles whose stencil lies in the window are counted per cell; the
+    // others (and, in mixed precision, values outside the window's range) go
+    // straight to HBM.
+    int cell[2], rank[2];
+    int bx0 = WX, bx1 = -1, by0 = WY, by1 = -1;
 #pragma unroll
-                        for (int b = 0; b < 6; b++) {
-                            const double wa = ax[0] * ay[b], wb = bx[0] * by[b];
-#pragma unroll
-                            for (int q = 0; q < 4; q++)
-                                shared_fix_add(swl, swh, q * WSZ + row + b,
-                                               fma(sv[0][q], wa, fma(sv[1][q], wb, FIX_MAGIC)));
-                        }
-#pragma unroll
-                        for (int k = 0; k < 5; k++) { ax[k] = ax[k + 1]; bx[k] = bx[k + 1]; }
-                        row += WY;
-                    }
-                } else {
-                    if (cx[0] >= 0)
-                        deposit_fix_one<WX, WY>(swl, swh, g4, N, wx0, wy0, cx[0], cy[0], dxl[0],
-                                                dyl[0], sv[0]);
-                    if (cx[1] >= 0)
-                        deposit_fix_one<WX, WY>(swl, swh, g4, N, wx0, wy0, cx[1], cy[1], dxl[1],
-                                                dyl[1], sv[1]);
-                }
-            } else if (joint) {
-                // the rows of the stencil in a rolled loop (the x weights
-                // move down one register per row): a fifth of the code,
-                // which keeps the stage's hot path within the instruction
-                // cache
-                double ax[5], ay[5], bx[5], by[5];
-                weights4(dxl[0], ax); weights4(dyl[0], ay);
-                weights4(dxl[1], bx); weights4(dyl[1], by);
-                int row = lx * WY + ly;
-#pragma unroll 1
-                for (int a = 0; a < 5; a++) {
-                    const double xa = ax[0], xb = bx[0];
-#pragma unroll
-                    for (int b = 0; b < 5; b++) {
-                        const double wa = xa * ay[b], wb = xb * by[b];
-#pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            shared_fix_add(swl, swh, q * WSZ + row + b,
-                                           fma(sv[0][q], wa, fma(sv[1][q], wb, FIX_MAGIC)));
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++) { ax[k] = ax[k + 1]; bx[k] = bx[k + 1]; }
-                    row += WY;
-                }
-            }
+    for (int p = 0; p < 2; p++) {
+        cell[p] = -1;
+        if (cx[p] < 0) continue;
+        const int lx = cx[p] - 2 - wx0, ly = cy[p] - 2 - wy0;
+        if (lx >= 0 && lx + 5 <= WX && ly >= 0 && ly + 5 <= WY && max_abs4(sv[p]) < (MIXED ? FIX_SHARED_LIMIT : 1e200)) {
+            cell[p] = ly * CX + lx;
+            rank[p] = atomicAdd(start + 1 + cell[p], 1);
+            bx0 = min(bx0, lx); bx1 = max(bx1, lx);
+            by0 = min(by0, ly); by1 = max(by1, ly);
+        } else {
+            deposit_direct<FT>(g4, N, cx[p], cy[p], dxl[p], dyl[p], sv[p]);
         }
-    } else {
-        const int lx = cx[0] - 2 - wx0, ly = cy[0] - 2 - wy0;
-        const bool joint = cx[0] >= 0 && cx[0] == cx[1] && cy[0] == cy[1] &&
-                           lx >= 0 && lx + 5 <= WX && ly >= 0 && ly + 5 <= WY;
-        double mj = 0;
+    }
+    bx0 = __reduce_min_sync(0xffffffffu, bx0);
+    bx1 = __reduce_max_sync(0xffffffffu, bx1);
+    by0 = __reduce_min_sync(0xffffffffu, by0);
+    by1 = __reduce_max_sync(0xffffffffu, by1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0 && bx1 >= 0) {
+        atomicMin(box, bx0); atomicMax(box + 1, bx1);
+        atomicMin(box + 2, by0); atomicMax(box + 3, by1);
+    }
+    __syncthreads();   // counts complete; the field window is read no more
+
+    // counts -> the cells' first records (start[c + 1] held cell c's count)
+    {
+        constexpr int E = (NC + THREADS - 1) / THREADS;
+        int n[E], sum = 0;
 #pragma unroll
-        for (int q = 0; q < 4; q++) mj = fmax(mj, fabs(sv[0][q]) + fabs(sv[1][q]));
-        const bool ok = mj * (0.36 * ih * ih) < FIX56_LIMIT;
-        if (!__all_sync(0xffffffffu, (joint && ok) || didle)) {
-            if (dpair && ok) {
-                double ax[6], ay[6], bx[6], by[6], t[5];
-                weights4(dxl[0], t); shift6(t, cx[0] - mcx, ax);
-                weights4(dyl[0], t); shift6(t, cy[0] - mcy, ay);
-                weights4(dxl[1], t); shift6(t, cx[1] - mcx, bx);
-                weights4(dyl[1], t); shift6(t, cy[1] - mcy, by);
+        for (int e = 0; e < E; e++) {
+            const int c = threadIdx.x * E + e;
+            n[e] = c < NC ? start[1 + c] : 0;
+            sum += n[e];
+        }
+        int incl = sum;
 #pragma unroll
-                for (int b = 0; b < 6; b++) { ay[b] *= ih; by[b] *= ih; }
-                int row = dx0 * WY + dy0;
-#pragma unroll 1
-                for (int a = 0; a < 6; a++) {
-                    const double xa = ax[0] * ih, xb = bx[0] * ih;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int at = incl - sum;
 #pragma unroll
-                    for (int b = 0; b < 6; b++) {
-                        const double wa = xa * ay[b], wb = xb * by[b];
+        for (int w = 0; w < THREADS / 32; w++)
+            if (w < warp) at += wsum[w];
 #pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            fix56_add(swl, sw1, sw2, q * WSZ + row + b, fma(sv[0][q], wa, sv[1][q] * wb));
-                    }
-#pragma unroll
-                    for (int k = 0; k < 5; k++) { ax[k] = ax[k + 1]; bx[k] = bx[k + 1]; }
-                    row += WY;
-                }
-            } else {
-#pragma unroll
-                for (int p = 0; p < 2; p++)
-                    if (cx[p] >= 0)
-                        deposit_fix56_one<WX, WY>(swl, sw1, sw2, g4, N, ih, wx0, wy0, cx[p], cy[p],
-                                                  dxl[p], dyl[p], sv[p]);
-            }
-        } else if (joint && ok) {
-            // the two contributions summed before the fixed-point atomics;
-            // the rows of the stencil in a rolled loop (the x weights move
-            // down one register per row): a fifth of the code, which keeps
-            // the stage's hot path within the instruction cache
-            double ax[5], ay[5], bx[5], by[5];
-            weights4(dxl[0], ax); weights4(dyl[0], ay);
-            weights4(dxl[1], bx); weights4(dyl[1], by);
-#pragma unroll
-            for (int b = 0; b < 5; b++) { ay[b] *= ih; by[b] *= ih; }
-            int row = lx * WY + ly;
-#pragma unroll 1
-            for (int a = 0; a < 5; a++) {
-                const double xa = ax[0] * ih, xb = bx[0] * ih;
-#pragma unroll
-                for (int b = 0; b < 5; b++) {
-                    const double wa = xa * ay[b], wb = xb * by[b];
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        fix56_add(swl, sw1, sw2, q * WSZ + row + b, fma(sv[0][q], wa, sv[1][q] * wb));
-                }
-#pragma unroll
-                for (int k = 0; k < 4; k++) { ax[k] = ax[k + 1]; bx[k] = bx[k + 1]; }
-                row += WY;
-            }
+        for (int e = 0; e < E; e++) {
+            const int c = threadIdx.x * E + e;
+            at += n[e];
+            if (c < NC) start[1 + c] = at;
         }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < WSZ; t += blockDim.x) {
-        const int gx = wx0 + t / WY, gy = wy0 + t % WY;
-        if (gx < 0 || gx >= N || gy < 0 || gy >= N) continue;
-        const int64_t c = (int64_t)gx * N + gy;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if constexpr (MIXED) {
-                const long long v = ((long long)swh[q * WSZ + t] << 20) + (long long)swl[q * WSZ + t];
-                if (v) atomicAdd(g4[q] + c, (fix_t)v);
-            } else {
-                const int i = q * WSZ + t;
-                if (swl[i] | sw1[i] | (unsigned)sw2[i])
-                    atomicAdd(g4[q] + c, fix56_value(swl[i], sw1[i], sw2[i]));
+    for (int p = 0; p < 2; p++) {
+        if (cell[p] < 0) continue;
+        double w[10];
+        weights4(dxl[p], w);
+        weights4(dyl[p], w + 5);
+        const int ly = cell[p] / CX, k = start[cell[p]] + rank[p] + ly;
+        double2 *r = reinterpret_cast<double2 *>(rec + k * S::RECORD);
+#pragma unroll
+        for (int u = 0; u < 5; u++) r[u] = make_double2(w[2 * u], w[2 * u + 1]);
+        r[5] = make_double2(sv[p][0], sv[p][1]);
+        r[6] = make_double2(sv[p][2], sv[p][3]);
+    }
+    __syncthreads();
+
+    // A lane takes XU cells along x and one quantity: the node sums of their
+    // particles in registers, then to HBM.  Neighbouring lanes take the four
+    // quantities (reading the same records), then the next column; the block's
+    // lanes share out the box of cells in use.
+    // mixed: a sum starts at FIX_MAGIC, where a unit in the last place is one,
+    // so that every term is rounded to an integer as it is added.
+    constexpr double ZERO = MIXED ? FIX_MAGIC : 0.0;
+    constexpr int XU = S::XU;
+    const int cx0 = box[0], nx = box[1] - cx0 + 1, cy0 = box[2], ny = box[3] - cy0 + 1;
+    if (ny <= 0) return;
+    const int q = threadIdx.x & 3;
+    Acc *const gq = q == 0 ? g4[0] : q == 1 ? g4[1] : q == 2 ? g4[2] : g4[3];
+    for (int u = threadIdx.x >> 2; u < ny * ((nx + XU - 1) / XU); u += THREADS / 4) {
+        const int ux = u / ny, c = cy0 + u - ux * ny, x = cx0 + ux * XU;
+        const int *col = start + c * CX + x;
+        double acc[XU + 4][5];
+#pragma unroll
+        for (int a = 0; a < XU + 4; a++)
+#pragma unroll
+            for (int b = 0; b < 5; b++) acc[a][b] = ZERO;
+        int k = col[0];
+#pragma unroll
+        for (int i = 0; i < XU; i++) {
+            const int end = x + i < CX ? col[i + 1] : k;
+            for (; k < end; k++) {
+                const double *r = rec + (k + c) * S::RECORD;
+                double w[10], t[5];
+#pragma unroll
+                for (int u = 0; u < 5; u++) {
+                    const double2 d = reinterpret_cast<const double2 *>(r)[u];
+                    w[2 * u] = d.x;
+                    w[2 * u + 1] = d.y;
+                }
+                const double v = r[10 + q], *wx = w;
+#pragma unroll
+                for (int b = 0; b < 5; b++) t[b] = w[5 + b] * v;
+#pragma unroll
+                for (int a = 0; a < 5; a++)
+#pragma unroll
+                    for (int b = 0; b < 5; b++) acc[a + i][b] = fma(wx[a], t[b], acc[a + i][b]);
             }
+        }
+        Acc *out = gq + (int64_t)(wx0 + x) * N + wy0 + c;
+#pragma unroll
+        for (int a = 0; a < XU + 4; a++) {
+#pragma unroll
+            for (int b = 0; b < 5; b++) {
+                const double t = acc[a][b];
+                if (t != ZERO) {
+                    if constexpr (MIXED) atomicAdd(out + b, fix_bits(t));
+                    else atomicAdd(out + b, t);
+                }
+            }
+            out += N;
         }
     }
 }
 
-template <typename FT, int WX, int WY>
-static size_t move_deposit_pair_smem()
-{
-    // deposit window: two 32-bit words per sum (mixed), three (FP64)
-    return (size_t)WX * WY * (FieldWin<FT>::bytes_per_cell + 4 * 4 * (sizeof(FT) == 4 ? 2 : 3));
-}
-
-template <typename FT, int WX, int WY, bool FIRST>
-static int launch_move_deposit_pair(const lcb_move_deposit_args *a, dim3 grid,
+template <typename S, typename FT, bool FIRST>
+static int launch_move_deposit(const lcb_move_deposit_args *a,
                                     typename StageAcc<FT>::type *const out[4], cudaStream_t st)
 {
-    const size_t sm = move_deposit_pair_smem<FT, WX, WY>();
+    const dim3 grid((a->particles_side + S::TJ - 1) / S::TJ,
+                    (a->particles_side + 1 + S::TI - 1) / S::TI,   // spare tile row
+                    a->n_sorts);
     static std::atomic<unsigned long long> attr{0};
     {
-        const cudaError_t e = ensure_smem(k_move_deposit_pair<FT, WX, WY, FIRST>, sm, attr);
+        const cudaError_t e = ensure_smem(k_move_deposit<S, FT, FIRST>, S::smem, attr);
         if (e != cudaSuccess) return cuda_check(e, "move_deposit smem attribute");
     }
     const lcb_plasma_particles &p = a->prev, &f = a->full;
     const cudaError_t e = launch_after(
-        k_move_deposit_pair<FT, WX, WY, FIRST>, grid, dim3(DEP_THREADS), sm, st,
-        a->n_per_sort, a->particles_side, a->grid_steps, a->h, a->xi_step, a->boundary,
+        k_move_deposit<S, FT, FIRST>, grid, dim3(S::THREADS), S::smem, st,
+        a->n_per_sort, a->particles_side, a->grid_steps, a->lattice_fineness, a->h, a->xi_step, a->boundary,
         a->fields[0], a->fields[1], a->fields[2], a->fields[3], a->fields[4], a->fields[5],
         p.x_init, p.y_init, p.x_offt, p.y_offt, p.px, p.py, p.pz, p.q, p.m,
         f.q, f.x_offt, f.y_offt, f.px, f.py, f.pz, out[0], out[1], out[2], out[3], a->err);
@@ -1234,20 +1163,19 @@ static int launch_move_deposit_pair(const lcb_move_deposit_args *a, dim3 grid,
     return LCB_OK;
 }
 
-// Window: the tile's cells (8 x 16 with two or more particles per cell,
-// 16 x 32 with one) + 2 stencil + 4 slack on each side.
+// Window: the tile's cells (8 x TJ / 2 with two or more particles per cell,
+// 16 x TJ with one) + 2 stencil + 4 slack on each side.
 template <typename FT>
-static int dispatch_move_deposit_pair(const lcb_move_deposit_args *a,
+static int dispatch_move_deposit(const lcb_move_deposit_args *a,
                                       typename StageAcc<FT>::type *const out[4], cudaStream_t st)
 {
-    const dim3 grid((a->particles_side + DEP_TJ - 1) / DEP_TJ,
-                    (a->particles_side + 1 + DEP_TI - 1) / DEP_TI,   // spare tile row
-                    a->n_sorts);
+    typedef Stage<FT, 20, 28> Two;
+    typedef Stage<FT, 28, 44> One;
     if (a->lattice_fineness >= 2)
-        return a->first ? launch_move_deposit_pair<FT, 20, 28, true>(a, grid, out, st)
-                        : launch_move_deposit_pair<FT, 20, 28, false>(a, grid, out, st);
-    return a->first ? launch_move_deposit_pair<FT, DEP_WX, DEP_WY, true>(a, grid, out, st)
-                    : launch_move_deposit_pair<FT, DEP_WX, DEP_WY, false>(a, grid, out, st);
+        return a->first ? launch_move_deposit<Two, FT, true>(a, out, st)
+                        : launch_move_deposit<Two, FT, false>(a, out, st);
+    return a->first ? launch_move_deposit<One, FT, true>(a, out, st)
+                    : launch_move_deposit<One, FT, false>(a, out, st);
 }
 
 // Fixed-point sums (4 quantities x 2 columns x N*N) to the FP64 outputs;
@@ -1276,10 +1204,11 @@ __global__ void k_fix_finish(int64_t plane, int n_sorts, const fix_t *__restrict
     }
 }
 
-// Zero four regions of n 8-byte words each (one kernel in the stream's chain
-// of programmatic launches, where a memset would break it).
+// Zero four regions of n 8-byte words each, or set the second half of the
+// first to `background` (one kernel in the stream's chain of programmatic
+// launches, where a memset or a copy would break it).
 __global__ void __launch_bounds__(256) k_zero4(uint64_t *r0, uint64_t *r1, uint64_t *r2, uint64_t *r3,
-                                               int64_t n)
+                                               const uint64_t *background, int64_t n)
 {
     pdl_wait();
     pdl_trigger();
@@ -1287,17 +1216,20 @@ __global__ void __launch_bounds__(256) k_zero4(uint64_t *r0, uint64_t *r1, uint6
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) r[q][t] = 0ull;
+        for (int q = 0; q < 4; q++)
+            r[q][t] = q == 0 && background && t >= n / 2 ? background[t - n / 2] : 0ull;
     }
 }
 
 static int grid_for(int64_t n, int threads);
 
-static int zero4(void *r0, void *r1, void *r2, void *r3, int64_t n, cudaStream_t st)
+static int zero4(void *r0, void *r1, void *r2, void *r3, int64_t n, cudaStream_t st,
+                 const double *background = nullptr)
 {
     const cudaError_t e = launch_after(k_zero4, dim3(grid_for(n, 256)), dim3(256), 0, st,
                                        static_cast<uint64_t *>(r0), static_cast<uint64_t *>(r1),
-                                       static_cast<uint64_t *>(r2), static_cast<uint64_t *>(r3), n);
+                                       static_cast<uint64_t *>(r2), static_cast<uint64_t *>(r3),
+                                       reinterpret_cast<const uint64_t *>(background), n);
     if (e != cudaSuccess) return cuda_check(e, "zero launch");
     count_launch();
     return LCB_OK;
@@ -1470,9 +1402,9 @@ extern "C" int lcb_plasma_move_deposit(const lcb_move_deposit_args *a, void *str
         if (rc0) return rc0;
         if (a->n_per_sort > 0) {
             fix_t *const out[4] = {w, w + 2 * plane, w + 4 * plane, w + 6 * plane};
-            const int rc = dispatch_move_deposit_pair<float>(a, out, st);
+            const int rc = dispatch_move_deposit<float>(a, out, st);
             if (rc) return rc;
-            LCB_LAUNCH_CHECK("k_move_deposit_pair<float>");
+            LCB_LAUNCH_CHECK("k_move_deposit<float>");
         }
         const cudaError_t e = launch_after(k_fix_finish, dim3(grid_for(plane, 256)), dim3(256), 0, st,
                                            (int64_t)plane, a->n_sorts, (const fix_t *)w,
@@ -1482,16 +1414,18 @@ extern "C" int lcb_plasma_move_deposit(const lcb_move_deposit_args *a, void *str
         return LCB_OK;
     }
     {
-        const int rc0 = zero4(a->ro, a->jx, a->jy, a->jz, 2 * (int64_t)plane, st);
+        // background ions go to the plane that no sort deposits into
+        const int rc0 = zero4(a->ro, a->jx, a->jy, a->jz, 2 * (int64_t)plane, st,
+                              a->n_sorts == 1 ? a->ro_initial : nullptr);
         if (rc0) return rc0;
     }
     if (a->n_per_sort > 0) {
         double *const out[4] = {a->ro, a->jx, a->jy, a->jz};
-        const int rc = dispatch_move_deposit_pair<double>(a, out, st);
+        const int rc = dispatch_move_deposit<double>(a, out, st);
         if (rc) return rc;
-        LCB_LAUNCH_CHECK("k_move_deposit_pair<double>");
+        LCB_LAUNCH_CHECK("k_move_deposit<double>");
     }
-    if (a->ro_initial) {
+    if (a->ro_initial && a->n_sorts > 1) {
         cudaError_t e = cudaMemcpyAsync(a->ro + plane, a->ro_initial, plane * sizeof(double),
                                         cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return cuda_check(e, "copy ro_initial");

@@ -1,0 +1,108 @@
+"""The fused particle stage against the three kernels run separately, where its
+tiles and rules can go wrong: one to four particles per cell along an axis
+(tiles of 16 x 32 particles cover 4 to 16 cells, odd sides leave remainders),
+one and two sorts, first and later stages, lattices that are not where the
+kernel expects the package's own (shifted by a cell and by half a cell), a
+lattice smaller than one tile, and a particle that is not a number.
+
+FP64: a node's sum has at most a few hundred terms of the same magnitude, so
+its rounding stays below 1e-13 of the largest; mixed: the gather's FP32
+weights and fields (6e-8 each) move the particles' momenta by at most that
+share of the fields' kick, far below 1e-5 of the currents."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover
+    pytest.skip("needs CUDA", allow_module_level=True)
+
+from lcodepy_b200 import _lib  # noqa: E402
+from lcodepy_b200.config import Config  # noqa: E402
+from lcodepy_b200.solver import CurrentSet, Plane2d3vPlasmaSolver  # noqa: E402
+
+DEV = torch.device("cuda")
+NAMES = ("x_offt", "y_offt", "px", "py", "pz", "q")
+
+
+def _solver(N, ppc, ion_model, precision, shift=0.0, seed=5):
+    h = 0.1
+    cfg = Config({'geometry': '3d', 'window-width': (N + 0.5) * h / 2, 'transverse-step': h, 'xi-step': h,
+                  'window-length': 1.0, 'ion-model': ion_model, 'plasma-particles-per-cell': ppc,
+                  'precision': precision, 'print-every': 0})
+    cfg._adjust_config_values_3d()
+    ps = Plane2d3vPlasmaSolver(cfg, DEV)
+    ps.init_state(0.0)
+    prev, full = ps.states
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+
+    def rnd(scale):
+        return (torch.rand(prev.q.numel(), generator=g, device=DEV, dtype=torch.float64) - 0.5) * 2 * scale
+    for s in (prev, full):
+        s.x_init += shift * h
+        s.y_init += shift * h
+    prev.x_offt.copy_(rnd(0.8 * h))
+    prev.y_offt.copy_(rnd(0.8 * h))
+    for k in ("px", "py", "pz"):
+        getattr(prev, k).copy_(rnd(0.3) * prev.m)
+    prev.q[::37] = 0        # absorbed earlier
+    for k in NAMES:
+        getattr(full, k).copy_(getattr(prev, k))
+    full.x_offt += rnd(0.05 * h)
+    full.y_offt += rnd(0.05 * h)
+    ps.fields[0].buf.copy_((torch.rand(7, ps.N, ps.N, generator=g, device=DEV, dtype=torch.float64) - 0.5) * 0.1)
+    return ps
+
+
+def _close(got, ref, rel, what):
+    scale = float(ref.abs().max())
+    assert float((got - ref).abs().max()) <= rel * max(scale, 1e-300), what
+
+
+@pytest.mark.parametrize("precision,rel", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("N,ppc,ions,first,shift", [
+    (65, 1, "background", True, 0.0), (65, 4, "background", False, 0.0), (67, 9, "mobile", False, 0.0),
+    (55, 16, "background", True, 0.0), (65, 4, "mobile", True, 1.0), (65, 4, "background", True, 0.5),
+    (65, 1, "background", False, -2.25), (33, 4, "background", True, 0.0)])
+def test_stage_against_separate_kernels(N, ppc, ions, first, shift, precision, rel):
+    ps = _solver(N, ppc, ions, precision, shift)
+    prev, full = ps.states
+    F = ps.fields[0]
+    start = {k: getattr(full, k).clone() for k in NAMES}
+    if first:
+        ps._move_wo_fields(prev, full)
+    ps._move_smart(F, prev, full)
+    want = CurrentSet(ps.N, DEV)
+    ps._deposit(full, want)
+    sep = {k: getattr(full, k).clone() for k in NAMES}
+    got = []
+    for _ in range(2):
+        for k, v in start.items():
+            getattr(full, k).copy_(v)
+        out = CurrentSet(ps.N, DEV)
+        out.buf.fill_(7.0)
+        ps._move_deposit(F, prev, full, out, first)
+        got.append(out.buf)
+    torch.cuda.synchronize()
+    assert int(ps.err.item()) == 0
+    for k in NAMES:
+        _close(getattr(full, k), sep[k], rel, k)
+    for i, k in enumerate(("ro", "jx", "jy", "jz")):
+        _close(got[0][i], want.buf[i], rel, k)
+    if precision == "mixed":
+        assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_stage_drops_a_particle_that_is_not_a_number(precision):
+    ps = _solver(65, 4, "background", precision)
+    prev, full = ps.states
+    k = prev.n_per_sort // 2 + 11
+    prev.px[k] = float("nan")
+    out = CurrentSet(ps.N, DEV)
+    ps._move_deposit(ps.fields[0], prev, full, out, True)
+    torch.cuda.synchronize()
+    assert int(ps.err.item()) & _lib.DEVERR_PLASMA_STENCIL
+    assert np.isfinite(out.buf.cpu().numpy()).all()
