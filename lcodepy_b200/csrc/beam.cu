@@ -4,43 +4,58 @@
 
 namespace lcb {
 
+// A particle's 25-point stencil is shared by a group of eight lanes, five of
+// which take a row of it (along y) each: the layers of a beam are a few
+// thousand particles, which would leave most of the chip idle with one thread
+// each, and a thread with hundreds of loads or additions in sequence.
+constexpr int BEAM_GROUP = 8;
+
+struct LayoutArgs {
+    int64_t n;
+    int N;
+    double h, xi_step, xi_layer;
+    const double *x, *y, *xi, *q;
+    double *ro0, *ro1;
+    int *err;
+};
+
 // Beam density deposit (lcode/beam3d/weights.py:108-138, driver :152-163):
 // q * w4(x) w4(y) * xi_loc into ro0 and * (1 - xi_loc) into ro1.  Stencil
 // points are addressed by the flat index (iy+ky) + N (ix+kx) as in the
 // reference; points whose flat index leaves [0, N*N) are skipped and flagged.
-__global__ void __launch_bounds__(128)
-k_beam_deposit(int64_t n, int N, double h, double xi_step, double xi_layer,
-               const double *__restrict__ x, const double *__restrict__ y,
-               const double *__restrict__ xi, const double *__restrict__ q,
-               double *ro0, double *ro1, int *err)
+// Thread `first` of `threads`.
+__device__ __forceinline__ void layout(const LayoutArgs &l, int64_t first, int64_t threads)
 {
-    const int half_n = N / 2;
-    const int64_t NN = (int64_t)N * N;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        const double xi_loc = (xi_layer - xi[k]) / xi_step;
+    const int half_n = l.N / 2, a = (int)(first % BEAM_GROUP);
+    const int64_t NN = (int64_t)l.N * l.N;
+    if (a >= 5) return;
+    for (int64_t k = first / BEAM_GROUP; k < l.n; k += threads / BEAM_GROUP) {
+        const double xi_loc = (l.xi_layer - l.xi[k]) / l.xi_step;
         double xl, yl;
-        const int ix = cell_of(x[k] / h + 0.5, half_n, xl);
-        const int iy = cell_of(y[k] / h + 0.5, half_n, yl);
+        const int ix = cell_of(l.x[k] / l.h + 0.5, half_n, xl);
+        const int iy = cell_of(l.y[k] / l.h + 0.5, half_n, yl);
         double wx[5], wy[5];
         weights4(xl, wx);
         weights4(yl, wy);
-        const double qk = q[k];
+        const double wxa = a == 0 ? wx[0] : a == 1 ? wx[1] : a == 2 ? wx[2] : a == 3 ? wx[3] : wx[4];
+        const double qk = l.q[k];
         bool bad = false;
 #pragma unroll
-        for (int a = 0; a < 5; a++) {
-#pragma unroll
-            for (int b = 0; b < 5; b++) {
-                const double w = wx[a] * wy[b];
-                const double w0 = w * xi_loc, w1 = w * (1 - xi_loc);
-                const int64_t idx = (int64_t)(iy + b - 2) + (int64_t)N * (ix + a - 2);
-                if (idx < 0 || idx >= NN) { bad = true; continue; }
-                atomicAdd(ro0 + idx, qk * w0);
-                atomicAdd(ro1 + idx, qk * w1);
-            }
+        for (int b = 0; b < 5; b++) {
+            const double w = wxa * wy[b];
+            const double w0 = w * xi_loc, w1 = w * (1 - xi_loc);
+            const int64_t idx = (int64_t)(iy + b - 2) + (int64_t)l.N * (ix + a - 2);
+            if (idx < 0 || idx >= NN) { bad = true; continue; }
+            atomicAdd(l.ro0 + idx, qk * w0);
+            atomicAdd(l.ro1 + idx, qk * w1);
         }
-        if (bad && err) atomicOr(err, LCB_DEVERR_BEAM_STENCIL);
+        if (bad && l.err) atomicOr(l.err, LCB_DEVERR_BEAM_STENCIL);
     }
+}
+
+__global__ void __launch_bounds__(128) k_beam_deposit(LayoutArgs l)
+{
+    layout(l, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 // Substep size (lcode/beam3d/beam_calculator.py:28-46) and the driver's
@@ -63,6 +78,12 @@ __global__ void k_beam_substepping(int64_t n, const double *__restrict__ q_m,
     }
 }
 
+// Layers up to this size push with a group of lanes per particle, larger ones
+// with one thread each.  A layer step (push, compaction, layout) on a 257
+// grid, groups against single threads: 13.6 / 18.6 us for 833 particles, 25.6
+// / 31.8 us for 8,333, 78.8 / 76.9 us for 33,333.
+constexpr int64_t BEAM_GROUP_MAX = 16384;
+
 struct FieldPair {
     const double *k[6], *k1[6];  // Ex Ey Ez Bx By Bz at plane k and k+1
 };
@@ -76,7 +97,11 @@ struct PushParams {
 // weighted with w0 = xi_loc on plane k and w1 = 1 - xi_loc on plane k+1, as
 // the reference GPU kernel weights them.  Updates the state in place and
 // returns the flags 1 lost | 2 moved | 4 fell; the id is negated when lost.
-__device__ uint8_t push_particle(const PushParams &P, const FieldPair &F, double qm, double dt,
+// G lanes of a warp (1, or BEAM_GROUP with the same particle in all of them;
+// `sub`: the lane's place) share the gather, a row of the stencil each, and
+// go through the rest together.
+template <int G>
+__device__ uint8_t push_particle(int sub, const PushParams &P, const FieldPair &F, double qm, double dt,
                                  int64_t &r, int64_t &id, double &x, double &y, double &xi,
                                  double &px, double &py, double &pz, int *err)
 {
@@ -91,8 +116,11 @@ __device__ uint8_t push_particle(const PushParams &P, const FieldPair &F, double
     }
     while (r > 0) {
         double gm = sqrt(im * im + px * px + py * py + pz * pz);
-        const double xh = x + dt / 2. * (px / gm);
-        const double yh = y + dt / 2. * (py / gm);
+        // p / gm: the longitudinal one as a quotient (it is subtracted from 1),
+        // the others by the reciprocal; the same for the rotation's factors
+        double ig = rcp_nr(gm);
+        const double xh = x + dt / 2. * (px * ig);
+        const double yh = y + dt / 2. * (py * ig);
         const double xih = xi + dt / 2. * (pz / gm - 1);
         if (xih < P.xi_k1) { fell = true; break; }
         if (xh * xh + yh * yh >= P.r_max * P.r_max) {
@@ -108,13 +136,17 @@ __device__ uint8_t push_particle(const PushParams &P, const FieldPair &F, double
         weights4(xl, wx);
         weights4(yl, wy);
         double Ex = 0, Ey = 0, Ez = 0, Bx = 0, By = 0, Bz = 0;
+        // one row (G > 1: the lane's own), or all five
 #pragma unroll
-        for (int a = 0; a < 5; a++) {
+        for (int u = 0; u < (G > 1 ? 1 : 5); u++) {
+            const int a = G > 1 ? sub : u;
+            const double wxa = a == 0 ? wx[0] : a == 1 ? wx[1] : a == 2 ? wx[2] : a == 3 ? wx[3] : wx[4];
 #pragma unroll
             for (int b = 0; b < 5; b++) {
-                const double w = wx[a] * wy[b];
+                const double w = wxa * wy[b];
                 const double w0 = w * xi_loc, w1 = w * (1 - xi_loc);
                 const int64_t idx = (int64_t)(iy + b - 2) + (int64_t)P.N * (ix + a - 2);
+                if (a >= 5) continue;
                 if (idx < 0 || idx >= NN) { bad = true; continue; }
                 Ex += __ldg(F.k[0] + idx) * w0 + __ldg(F.k1[0] + idx) * w1;
                 Bx += __ldg(F.k[3] + idx) * w0 + __ldg(F.k1[3] + idx) * w1;
@@ -122,6 +154,15 @@ __device__ uint8_t push_particle(const PushParams &P, const FieldPair &F, double
                 By += __ldg(F.k[4] + idx) * w0 + __ldg(F.k1[4] + idx) * w1;
                 Ez += __ldg(F.k[2] + idx) * w0 + __ldg(F.k1[2] + idx) * w1;
                 Bz += __ldg(F.k[5] + idx) * w0 + __ldg(F.k1[5] + idx) * w1;
+            }
+        }
+        if (G > 1) {
+            const unsigned lanes = ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) / G * G);
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+                Ex += __shfl_xor_sync(lanes, Ex, o); Bx += __shfl_xor_sync(lanes, Bx, o);
+                Ey += __shfl_xor_sync(lanes, Ey, o); By += __shfl_xor_sync(lanes, By, o);
+                Ez += __shfl_xor_sync(lanes, Ez, o); Bz += __shfl_xor_sync(lanes, Bz, o);
             }
         }
         const double hd = q * dt / 2.;
@@ -133,17 +174,20 @@ __device__ uint8_t push_particle(const PushParams &P, const FieldPair &F, double
         const double bp = bx * pxm + by * pym + bz * pzm;
         const double g2 = gm * gm - bsq;
         gm = sqrt((g2 + sqrt(g2 * g2 + 4 * bsq + 4 * bp * bp)) / 2.);
-        const double tx = bx / gm, ty = by / gm, tz = bz / gm;
+        ig = rcp_nr(gm);
+        const double tx = bx * ig, ty = by * ig, tz = bz * ig;
         const double tp = 1. + tx * tx + ty * ty + tz * tz;
         const double tmn = 1. - tx * tx - ty * ty - tz * tz;
-        const double sx = 2. * tx / tp, sy = 2. * ty / tp, sz = 2. * tz / tp;
+        const double itp = rcp_nr(tp), mix = tmn * itp;
+        const double sx = 2. * tx * itp, sy = 2. * ty * itp, sz = 2. * tz * itp;
         const double sp = sx * pxm + sy * pym + sz * pzm;
-        px = tx * sp + pxm * tmn / tp + pym * sz - pzm * sy + hd * Ex;
-        py = ty * sp + pym * tmn / tp + pzm * sx - pxm * sz + hd * Ey;
-        pz = tz * sp + pzm * tmn / tp + pxm * sy - pym * sx + hd * Ez;
+        px = tx * sp + pxm * mix + pym * sz - pzm * sy + hd * Ex;
+        py = ty * sp + pym * mix + pzm * sx - pxm * sz + hd * Ey;
+        pz = tz * sp + pzm * mix + pxm * sy - pym * sx + hd * Ez;
         gm = sqrt(im * im + px * px + py * py + pz * pz);
-        x = xh + dt / 2. * (px / gm);
-        y = yh + dt / 2. * (py / gm);
+        ig = rcp_nr(gm);
+        x = xh + dt / 2. * (px * ig);
+        y = yh + dt / 2. * (py * ig);
         xi = xih + dt / 2. * (pz / gm - 1);
         if (x * x + y * y >= P.r_max * P.r_max) { lost = true; r = 0; break; }
         r -= 1;
@@ -154,17 +198,22 @@ __device__ uint8_t push_particle(const PushParams &P, const FieldPair &F, double
     return (uint8_t)((lost ? 1 : 0) | (fell ? 4 : 0) | (!fell && !lost ? 2 : 0));
 }
 
+template <int G>
 __global__ void __launch_bounds__(128)
 k_beam_move(int64_t n, PushParams P, const double *__restrict__ q_m,
             const double *__restrict__ dt_a, FieldPair F, int64_t *rem,
             int64_t *id, double *xa, double *ya, double *xia, double *pxa,
             double *pya, double *pza, uint8_t *flags, int *err)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
+    const int sub = threadIdx.x % G;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G; i < n;
+         i += (int64_t)gridDim.x * blockDim.x / G) {
         double x = xa[i], y = ya[i], xi = xia[i], px = pxa[i], py = pya[i], pz = pza[i];
         int64_t r = rem[i], pid = id[i];
-        flags[i] = push_particle(P, F, q_m[i], dt_a[i], r, pid, x, y, xi, px, py, pz, err);
+        const uint8_t f = push_particle<G>(sub, P, F, q_m[i], dt_a[i], r, pid, x, y, xi, px, py, pz, err);
+        if (G > 1) __syncwarp(((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) / G * G));   // all have read it
+        if (sub != 0) continue;
+        flags[i] = f;
         xa[i] = x; ya[i] = y; xia[i] = xi; pxa[i] = px; pya[i] = py; pza[i] = pz;
         rem[i] = r;
         id[i] = pid;
@@ -199,6 +248,7 @@ struct StepArgs {
     FieldPair F;
     double *clear;          // plane zeroed by the same grid (the next layout's lower plane)
     int64_t clear_n;
+    int64_t *fell_out_count;   // zeroed too (the compaction's blocks check out there)
     int *err;
 };
 
@@ -220,14 +270,19 @@ __device__ __forceinline__ void soa_store(const lcb_beam_soa &s, int64_t i, cons
     s.remaining_steps[i] = rem;
 }
 
+template <int G>
 __global__ void __launch_bounds__(128) k_beam_push_stage(StepArgs a)
 {
+    pdl_wait();
+    pdl_trigger();
+    if (a.fell_out_count && blockIdx.x == 0 && threadIdx.x == 0) *a.fell_out_count = 0;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < a.clear_n;
          t += (int64_t)gridDim.x * blockDim.x)
         a.clear[t] = 0.0;
     const int64_t total = a.n_fresh + *a.fell_in_count;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
+    const int sub = threadIdx.x % G;
+    for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G; t < total;
+         t += (int64_t)gridDim.x * blockDim.x / G) {
         if (t >= a.stage_capacity) {
             if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
             break;
@@ -242,9 +297,12 @@ __global__ void __launch_bounds__(128) k_beam_push_stage(StepArgs a)
         } else {
             soa_load(a.fin, t - a.n_fresh, v, id, rem);
         }
-        a.flags[t] = push_particle(a.P, a.F, v[6], v[8], rem, id, v[1], v[2], v[0], v[3],
-                                   v[4], v[5], a.err);
-        soa_store(a.stage, t, v, id, rem);
+        const uint8_t f = push_particle<G>(sub, a.P, a.F, v[6], v[8], rem, id, v[1], v[2], v[0], v[3],
+                                           v[4], v[5], a.err);
+        if (sub == 0) {
+            a.flags[t] = f;
+            soa_store(a.stage, t, v, id, rem);
+        }
     }
 }
 
@@ -259,83 +317,118 @@ struct CompactArgs {
     int *err;
 };
 
-constexpr int CMP_THREADS = 1024;
+// Ordered compaction: a block takes tiles of 256 staged particles and finds
+// where a tile's particles go by counting the flags before it itself (a byte
+// per particle, from L2), so that the blocks do not wait for one another.
+// The counters may only move once every block has read them: the blocks check
+// out at fell_out_count, which the push has zeroed, and the last one writes
+// all three.  The grid's other blocks lay out the next layer meanwhile (that
+// reads only the source, and the push's grid has cleared ro1).
+// For a layer of 8,300 particles one block over all chunks took 34 us and the
+// layout another 9 after it.
+constexpr int CMP_THREADS = 256, CMP_WARPS = CMP_THREADS / 32;
 
-// Ordered compaction by one CTA: an exclusive scan of three 20-bit counters
-// packed in a 64-bit word per chunk of 1024 staged particles.
-__global__ void __launch_bounds__(CMP_THREADS) k_beam_compact(CompactArgs a)
+struct FlagCounts { int moved, fell, lost; };
+
+__device__ __forceinline__ void count_word(FlagCounts &c, unsigned w)
 {
-    __shared__ unsigned long long warp_sums[CMP_THREADS / 32];
-    __shared__ long long base[3];
+    c.moved += __popc(w & 0x02020202u);
+    c.fell += __popc(w & 0x04040404u);
+    c.lost += __popc(w & 0x01010101u);
+}
+
+// The block's sums over flags [from, to), the same in every thread.
+__device__ FlagCounts count_flags(const uint8_t *flags, int64_t from, int64_t to, int (*red)[3])
+{
+    FlagCounts c = {0, 0, 0};
+    const int tid = threadIdx.x;
+    int64_t k = from;
+    if (((uintptr_t)(flags + from) & 15) == 0) {
+        const int64_t quads = (to - from) / 16;
+        const uint4 *q = reinterpret_cast<const uint4 *>(flags + from);
+        for (int64_t t = tid; t < quads; t += CMP_THREADS) {
+            const uint4 w = q[t];
+            count_word(c, w.x); count_word(c, w.y); count_word(c, w.z); count_word(c, w.w);
+        }
+        k += quads * 16;
+    }
+    for (k += tid; k < to; k += CMP_THREADS) count_word(c, flags[k]);
+    c.moved = __reduce_add_sync(0xffffffffu, c.moved);
+    c.fell = __reduce_add_sync(0xffffffffu, c.fell);
+    c.lost = __reduce_add_sync(0xffffffffu, c.lost);
+    __syncthreads();   // the last sums have been read
+    if ((tid & 31) == 0) {
+        red[tid >> 5][0] = c.moved; red[tid >> 5][1] = c.fell; red[tid >> 5][2] = c.lost;
+    }
+    __syncthreads();
+    c = {0, 0, 0};
+#pragma unroll
+    for (int w = 0; w < CMP_WARPS; w++) {
+        c.moved += red[w][0]; c.fell += red[w][1]; c.lost += red[w][2];
+    }
+    return c;
+}
+
+__device__ void compact(const CompactArgs &a, int block, int blocks)
+{
+    __shared__ int red[CMP_WARPS][3], wsum[CMP_WARPS][3];
+    __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int64_t total = a.n_fresh + *a.fell_in_count;
     if (total > a.stage_capacity) total = a.stage_capacity;
+    const int64_t drain0 = *a.drain_count, lost0 = a.lost_count ? *a.lost_count : 0;
+    int64_t om = drain0, of = 0, ol = lost0, counted = 0;   // places of the tile's first ones
+    for (int64_t t0 = (int64_t)block * CMP_THREADS; t0 < total; t0 += (int64_t)blocks * CMP_THREADS) {
+        const FlagCounts before = count_flags(a.flags, counted, t0, red);
+        counted = t0;
+        om += before.moved; of += before.fell; ol += before.lost;
+        const int64_t t = t0 + tid;
+        const uint8_t f = t < total ? a.flags[t] : 0;
+        double v[9];
+        int64_t id = 0, rem = 0;
+        if (f) soa_load(a.stage, t, v, id, rem);
+        const unsigned mm = __ballot_sync(0xffffffffu, f & 2), mf = __ballot_sync(0xffffffffu, f & 4),
+                       ml = __ballot_sync(0xffffffffu, f & 1), lower = (1u << lane) - 1u;
+        if (lane == 0) { wsum[warp][0] = __popc(mm); wsum[warp][1] = __popc(mf); wsum[warp][2] = __popc(ml); }
+        __syncthreads();
+        int pm = __popc(mm & lower), pf = __popc(mf & lower), pl = __popc(ml & lower);
+        for (int w = 0; w < warp; w++) { pm += wsum[w][0]; pf += wsum[w][1]; pl += wsum[w][2]; }
+        if (f & 2) {
+            if (om + pm < a.drain_capacity) soa_store(a.drain, om + pm, v, id, rem);
+            else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
+        } else if (f & 4) {
+            if (of + pf < a.fell_capacity) soa_store(a.fout, of + pf, v, id, rem);
+            else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
+        } else if ((f & 1) && a.lost.id) {
+            if (ol + pl < a.lost_capacity) soa_store(a.lost, ol + pl, v, id, rem);
+            else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
+        }
+    }
+    __syncthreads();   // every thread has read the counters
     if (tid == 0) {
-        base[0] = *a.drain_count;
-        base[1] = 0;
-        base[2] = a.lost_count ? *a.lost_count : 0;
+        __threadfence();
+        last = blocks == 1 ||
+               atomicAdd(reinterpret_cast<unsigned long long *>(a.fell_out_count), 1ull) ==
+               (unsigned long long)(blocks - 1);
     }
     __syncthreads();
-    for (int64_t c0 = 0; c0 < total; c0 += CMP_THREADS) {
-        const int64_t t = c0 + tid;
-        const uint8_t f = t < total ? a.flags[t] : 0;
-        const unsigned long long mine = (unsigned long long)((f & 2) ? 1 : 0) |
-                                        ((unsigned long long)((f & 4) ? 1 : 0) << 20) |
-                                        ((unsigned long long)((f & 1) ? 1 : 0) << 40);
-        unsigned long long incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) warp_sums[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const unsigned long long v = warp_sums[lane];
-            unsigned long long s = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_up_sync(0xffffffffu, s, o);
-                if (lane >= o) s += y;
-            }
-            warp_sums[lane] = s - v;  // exclusive over warps
-        }
-        __syncthreads();
-        const unsigned long long excl = warp_sums[warp] + incl - mine;
-        const int64_t om = (int64_t)(excl & 0xFFFFF), ofl = (int64_t)((excl >> 20) & 0xFFFFF),
-                      ol = (int64_t)((excl >> 40) & 0xFFFFF);
-        if (t < total && f) {
-            double v[9];
-            int64_t id, rem;
-            soa_load(a.stage, t, v, id, rem);
-            if (f & 2) {
-                const int64_t dst = base[0] + om;
-                if (dst < a.drain_capacity) soa_store(a.drain, dst, v, id, rem);
-                else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
-            } else if (f & 4) {
-                const int64_t dst = base[1] + ofl;
-                if (dst < a.fell_capacity) soa_store(a.fout, dst, v, id, rem);
-                else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
-            } else if ((f & 1) && a.lost.id) {
-                const int64_t dst = base[2] + ol;
-                if (dst < a.lost_capacity) soa_store(a.lost, dst, v, id, rem);
-                else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
-            }
-        }
-        __syncthreads();
-        if (tid == CMP_THREADS - 1) {
-            const unsigned long long tot = excl + mine;
-            base[0] += (long long)(tot & 0xFFFFF);
-            base[1] += (long long)((tot >> 20) & 0xFFFFF);
-            base[2] += (long long)((tot >> 40) & 0xFFFFF);
-        }
-        __syncthreads();
-    }
+    if (!last) return;
+    const FlagCounts all = count_flags(a.flags, 0, total, red);
     if (tid == 0) {
-        *a.drain_count = base[0] < a.drain_capacity ? base[0] : a.drain_capacity;
-        *a.fell_out_count = base[1] < a.fell_capacity ? base[1] : a.fell_capacity;
-        if (a.lost_count) *a.lost_count = base[2] < a.lost_capacity ? base[2] : a.lost_capacity;
+        const int64_t d = drain0 + all.moved, l = lost0 + all.lost;
+        *a.drain_count = d < a.drain_capacity ? d : a.drain_capacity;
+        *a.fell_out_count = all.fell < a.fell_capacity ? all.fell : a.fell_capacity;
+        if (a.lost_count) *a.lost_count = l < a.lost_capacity ? l : a.lost_capacity;
     }
+}
+
+__global__ void __launch_bounds__(CMP_THREADS) k_beam_compact_layout(CompactArgs a, LayoutArgs l, int blocks)
+{
+    pdl_wait();
+    pdl_trigger();
+    if ((int)blockIdx.x < blocks) compact(a, blockIdx.x, blocks);
+    else layout(l, (int64_t)(blockIdx.x - blocks) * CMP_THREADS + threadIdx.x,
+                (int64_t)(gridDim.x - blocks) * CMP_THREADS);
 }
 
 static int grid_for(int64_t n, int threads)
@@ -357,9 +450,8 @@ extern "C" int lcb_beam_deposit(int64_t n, int grid_steps, double h, double xi_s
 {
     LCB_REQUIRE(n >= 0 && grid_steps >= 5, "bad sizes");
     if (n == 0) return LCB_OK;
-    const double xi_layer = -xi_step * (double)layer_idx;
-    k_beam_deposit<<<grid_for(n, 128), 128, 0, as_stream(stream)>>>(
-        n, grid_steps, h, xi_step, xi_layer, x, y, xi, q_norm, ro0, ro1, err);
+    const LayoutArgs l = {n, grid_steps, h, xi_step, -xi_step * (double)layer_idx, x, y, xi, q_norm, ro0, ro1, err};
+    k_beam_deposit<<<grid_for(n * BEAM_GROUP, 128), 128, 0, as_stream(stream)>>>(l);
     LCB_LAUNCH_CHECK("k_beam_deposit");
     return LCB_OK;
 }
@@ -398,8 +490,12 @@ extern "C" int lcb_beam_move(int64_t n, double xi_step, double r_max,
     P.xi_step = xi_step; P.r_max = r_max; P.h = h; P.N = grid_steps;
     P.xi_k = (double)beam_layer_idx * (-xi_step);
     P.xi_k1 = (double)(beam_layer_idx + 1) * (-xi_step);
-    k_beam_move<<<grid_for(n, 128), 128, 0, as_stream(stream)>>>(
-        n, P, q_m, dt, F, remaining_steps, id, x, y, xi, px, py, pz, flags, err);
+    if (n <= BEAM_GROUP_MAX)
+        k_beam_move<BEAM_GROUP><<<grid_for(n * BEAM_GROUP, 128), 128, 0, as_stream(stream)>>>(
+            n, P, q_m, dt, F, remaining_steps, id, x, y, xi, px, py, pz, flags, err);
+    else
+        k_beam_move<1><<<grid_for(n, 128), 128, 0, as_stream(stream)>>>(
+            n, P, q_m, dt, F, remaining_steps, id, x, y, xi, px, py, pz, flags, err);
     LCB_LAUNCH_CHECK("k_beam_move");
     return LCB_OK;
 }
@@ -445,9 +541,18 @@ extern "C" int lcb_beam_step(const lcb_beam_step_args *a, void *stream)
     }
     s.clear = a->ro1;
     s.clear_n = (int64_t)N * N;
+    // (one block compacts where the counter of the fallen is updated in place)
+    const bool in_place = a->fell_out_count == a->fell_in_count;
+    s.fell_out_count = in_place ? nullptr : a->fell_out_count;
     s.err = a->err;
-    k_beam_push_stage<<<2 * sm_count(), 128, 0, st>>>(s);
-    LCB_LAUNCH_CHECK("k_beam_push_stage");
+    // at least two blocks per SM, for the plane and for particles that fell
+    // (their number is on the device)
+    const bool group = s.n_fresh <= BEAM_GROUP_MAX;
+    const int pg = grid_for(group ? s.n_fresh * BEAM_GROUP : s.n_fresh, 128), most = 2 * sm_count();
+    cudaError_t e = launch_after(group ? k_beam_push_stage<BEAM_GROUP> : k_beam_push_stage<1>,
+                                 dim3(pg > most ? pg : most), dim3(128), 0, st, s);
+    if (e != cudaSuccess) return cuda_check(e, "beam push launch");
+    count_launch();
     CompactArgs c;
     c.stage = a->stage; c.drain = a->drain; c.fout = a->fell_out; c.lost = a->lost;
     c.flags = a->stage_flags;
@@ -458,16 +563,19 @@ extern "C" int lcb_beam_step(const lcb_beam_step_args *a, void *stream)
     c.drain_capacity = a->drain_capacity; c.fell_capacity = a->fell_capacity;
     c.lost_capacity = a->lost_capacity;
     c.err = a->err;
-    k_beam_compact<<<1, CMP_THREADS, 0, st>>>(c);
-    LCB_LAUNCH_CHECK("k_beam_compact");
-    // the layout reads only the source and ro1 was cleared by the push grid
-    if (a->layout_end > a->layout_begin) {
-        const int64_t n = a->layout_end - a->layout_begin, o = a->layout_begin;
-        k_beam_deposit<<<grid_for(n, 128), 128, 0, st>>>(
-            n, N, a->h, a->xi_step, -a->xi_step * (double)a->layout_idx,
-            a->source.x + o, a->source.y + o, a->source.xi + o, a->source.q_norm + o,
-            a->ro0, a->ro1, a->err);
-        LCB_LAUNCH_CHECK("k_beam_deposit");
-    }
+    const int64_t n = a->layout_end - a->layout_begin, o = a->layout_begin;
+    const LayoutArgs l = {n, N, a->h, a->xi_step, -a->xi_step * (double)a->layout_idx,
+                          a->source.x + o, a->source.y + o, a->source.xi + o, a->source.q_norm + o,
+                          a->ro0, a->ro1, a->err};
+    // one block per tile of fresh particles and one for those that fell, up to
+    // two per SM; as many again at most for the layout
+    auto blocks = [&](int64_t threads) {
+        const int64_t b = (threads + CMP_THREADS - 1) / CMP_THREADS;
+        return (int)(b < most ? b : most);
+    };
+    const int nc = in_place ? 1 : blocks(c.n_fresh + CMP_THREADS);
+    e = launch_after(k_beam_compact_layout, dim3(nc + blocks(n * BEAM_GROUP)), dim3(CMP_THREADS), 0, st, c, l, nc);
+    if (e != cudaSuccess) return cuda_check(e, "beam compaction launch");
+    count_launch();
     return LCB_OK;
 }

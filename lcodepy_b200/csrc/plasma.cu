@@ -586,29 +586,6 @@ template <typename FT> struct StageAcc;
 template <> struct StageAcc<float> { typedef fix_t type; };
 template <> struct StageAcc<double> { typedef double type; };
 
-// 1 / x and sqrt(x) for normal positive x by Newton's method from the
-// hardware's approximations (about 2^-20): a step of third order for the
-// reciprocal, two coupled second-order steps for the root, within two units
-// in the last place.  Shorter chains than the correctly rounded operations;
-// a stage has four to five of each per particle in sequence.
-__device__ __forceinline__ double rcp_nr(double x)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-__device__ __forceinline__ double sqrt_nr(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double g = x * y, h = 0.5 * y;
-    const double e = fma(-g, h, 0.5);
-    g = fma(g, e, g);
-    h = fma(h, e, h);
-    return fma(fma(-g, g, x), h, g);
-}
-
 // Shape of a block of the fused stage: TI x TJ lattice particles, two per
 // thread; a window of WX x WY nodes around them.
 template <typename FT, int WX_, int WY_> struct Stage {

@@ -1,0 +1,107 @@
+"""One layer step of the beam against its parts: the push by lcb_beam_move and
+the ordered selection of moved, fallen and lost particles by boolean masks, at
+the edges of the compaction's tiles (256 particles), in both forms of the push
+(a group of lanes per particle up to 16384, a thread each above) and with the
+fallen particles' counter updated in place."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover
+    pytest.skip("needs CUDA", allow_module_level=True)
+
+from lcodepy_b200 import _lib  # noqa: E402
+from lcodepy_b200.beam3d import BeamCalculator, BeamParticles, BeamSource  # noqa: E402
+from lcodepy_b200.config import Config  # noqa: E402
+
+DEV = torch.device("cuda")
+STATE = ("xi", "x", "y", "px", "py", "pz")
+
+
+class Planes:
+    def __init__(self, buf):
+        self.buf = buf
+        self.struct = _lib.Fields7()
+        for i in range(7):
+            self.struct.f[i] = buf[i].data_ptr()
+
+
+def _beam(n, layer, dxi, g):
+    """Particles of one layer: fast ones, slow ones that fall behind, and some
+    near the radius where they are lost."""
+    def rnd():
+        return torch.rand(n, generator=g, device=DEV, dtype=torch.float64)
+    b = BeamParticles(DEV)
+    b.xi = torch.sort(-dxi * (layer + rnd().clamp(1e-3, 1 - 1e-3)), descending=True).values
+    b.x, b.y = rnd() * 2.3 - 1.15, rnd() * 2.3 - 1.15
+    b.px, b.py = rnd() - 0.5, rnd() - 0.5
+    b.pz = torch.where(rnd() < 0.4, 0.8 + 2 * rnd(), 1000 + rnd())
+    b.q_m = -torch.ones_like(b.xi)
+    b.q_norm = rnd()
+    b.id = torch.arange(1, n + 1, device=DEV, dtype=torch.int64)
+    b.dt = torch.zeros_like(b.xi)
+    b.remaining_steps = torch.zeros_like(b.id)
+    return b
+
+
+@pytest.mark.parametrize("n,in_place", [(1, False), (255, False), (256, False), (257, False), (5000, False),
+                                        (5000, True), (20000, False)])
+def test_layer_step_against_its_parts(n, in_place):
+    L = _lib.load()
+    N, dxi = 65, 0.05
+    cfg = Config({'geometry': '3d', 'window-width': 1.63, 'transverse-step': 0.05, 'window-length': 1.0,
+                  'xi-step': dxi, 'time-step': 1.0})
+    cfg._adjust_config_values_3d()
+    assert cfg.getint('window-width-steps') == N
+    g = torch.Generator(device=DEV)
+    g.manual_seed(n)
+    layer = 3
+    b = _beam(n, layer, dxi, g)
+    F = [Planes((torch.rand(7, N, N, generator=g, device=DEV, dtype=torch.float64) - 0.5) * 0.4) for _ in range(2)]
+    bc = BeamCalculator(cfg, DEV)
+    bc.start_time_step(BeamSource(cfg, b, DEV))
+    if in_place:
+        bc.counts = torch.zeros_like(bc.counts)
+        a = bc._args(layer + 1, (0, 0), (0, n), F[0], F[1])
+        a.fell_out_count = a.fell_in_count
+    else:
+        a = bc._args(layer + 1, (0, 0), (0, n), F[0], F[1])
+    bc.drain.id[:] = -7
+    _lib.check(L.lcb_beam_step(C.byref(a), _lib.stream_handle()), "lcb_beam_step")
+
+    dt, rs = torch.zeros_like(b.xi), torch.zeros_like(b.id)
+    st = _lib.stream_handle()
+    _lib.check(L.lcb_beam_substepping(n, b.q_m.data_ptr(), b.pz.data_ptr(), 2.0, 1.0, dt.data_ptr(), rs.data_ptr(),
+                                      st), "substepping")
+    p = {k: getattr(b, k).clone() for k in STATE}
+    ids = b.id.clone()
+    flags = torch.zeros(n, dtype=torch.uint8, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    _lib.check(L.lcb_beam_move(n, dxi, bc.r_max, layer, bc.h, N, b.q_m.data_ptr(), dt.data_ptr(),
+                               C.byref(F[0].struct), C.byref(F[1].struct), rs.data_ptr(), ids.data_ptr(),
+                               *(p[k].data_ptr() for k in ("x", "y", "xi", "px", "py", "pz")), flags.data_ptr(),
+                               err.data_ptr(), st), "lcb_beam_move")
+    torch.cuda.synchronize()
+    f = flags.cpu().numpy()
+    counts = bc.counts.cpu().numpy()
+    fell_slot = bc.fell_cur if in_place else 1 - bc.fell_cur
+    moved, fell = (f & 2) > 0, (f & 4) > 0
+    assert n < 200 or (moved.any() and fell.any() and (f & 1).any())
+    assert counts[2] == moved.sum() and counts[fell_slot] == fell.sum() and counts[3] == ((f & 1) > 0).sum()
+    for buf, mask in ((bc.drain, moved), (bc.fell[1 - bc.fell_cur], fell)):
+        k = int(mask.sum())
+        np.testing.assert_array_equal(buf.id[:k].cpu().numpy(), ids.cpu().numpy()[mask])
+        np.testing.assert_array_equal(buf.remaining_steps[:k].cpu().numpy(), rs.cpu().numpy()[mask])
+        for name in STATE:
+            np.testing.assert_array_equal(getattr(buf, name)[:k].cpu().numpy(), p[name].cpu().numpy()[mask])
+    # the lost ones that did not fall sit at their rank among all lost ones
+    lost = (f & 1) > 0
+    at = np.cumsum(lost) - 1
+    only = lost & ~fell
+    np.testing.assert_array_equal(bc.lost.id.cpu().numpy()[at[only]], ids.cpu().numpy()[only])
+    if n > 1:
+        assert (bc.drain.id[int(moved.sum()):] == -7).all()
