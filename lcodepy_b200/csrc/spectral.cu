@@ -32,15 +32,21 @@
 // 6.65 TB/s), the transforms 0.2 GFLOP of FP64.  As dense products on the
 // tensor cores (fields.cu, exact int8 slices) the same solve took 187 us in
 // FP64 and 105 us in mixed precision (without Phi), against 54.5 and 50 us
-// here: 36 slice products per multiply-add and N multiply-adds per node and
-// transform cost more than log N FP64 operations on the vector units.  At 129
-// the solve went from 62.9 to 31.6 us (four launches instead of eleven), at
-// 331, with the kernels for any length, from 83.9 to 51.6 us.  The error
+// with these kernels at first and 50 and 44 us now: 36 slice products per
+// multiply-add and N multiply-adds per node and transform cost more than log N
+// FP64 operations on the vector units.  At 129 the solve went from 62.9 to
+// 31.6 us (four launches instead of eleven), at 331, with the kernels for any
+// length, from 83.9 to 47 us.  Of the 50 us (cold, each by itself) the
+// right-hand sides take 15, the rows 10, the columns 17.5 and the rows back 14:
+// latency at 16 warps per SM, the L2's 32-byte sectors in the columns.  The error
 // against 64-bit sums is 6e-16 (dense: 1e-14 FP64, 1e-6 mixed, at 513).
 //
 // Rounding of one field reaches the others of its unit at 2^-53 of the
 // largest of them; the right-hand sides of a unit are differences of the same
 // densities and carry the rounding of those already.
+#include <map>
+#include <mutex>
+
 #include "dft.cuh"
 #include "spectral.cuh"
 
@@ -138,6 +144,7 @@ struct OpsView {
 
 static size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 
+// The plan of a grid, found once per size (a solve asks for it on every call).
 static bool plan_of(int N, DftPlan &p)
 {
     const int L = 2 * (N - 1), q = fixed_q(L);
@@ -147,7 +154,17 @@ static bool plan_of(int N, DftPlan &p)
         plan_offsets(p);
         return true;
     }
-    return make_plan(L, p);
+    static std::mutex mu;
+    static std::map<int, DftPlan> plans;   // n = 0: the size has none
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = plans.find(L);
+    if (it == plans.end()) {
+        DftPlan made;
+        if (!make_plan(L, made)) made.n = 0;
+        it = plans.emplace(L, made).first;
+    }
+    p = it->second;
+    return p.n > 0;
 }
 
 static OpsView ops_view(const void *ops, int N, const DftPlan &p)
@@ -168,10 +185,9 @@ static size_t any_smem(int L, int cols) { return (size_t)cols * 2 * sp_line(L) *
 
 bool spectral_grid(int N)
 {
-    if (N < 5 || N % 2 == 0) return false;
+    if (N < 5 || N % 2 == 0 || N > 8192 || any_smem(2 * (N - 1), 1) > 220 * 1024) return false;
     DftPlan p;
-    if (!plan_of(N, p)) return false;
-    return any_smem(p.L, 1) <= 220 * 1024;
+    return plan_of(N, p);
 }
 
 size_t spectral_ops_bytes(int N)
@@ -582,6 +598,10 @@ template <int Q> struct Fix {
     static constexpr int B = 8 * Q;    // radix-8 butterflies of a step (two per thread)
 };
 
+// Element b + q B of a line of length 8 B is one of the first half (up to M =
+// 4 B), or else the mirror image of element (B - b) + (7 - q) B.
+__device__ __forceinline__ bool fix_direct(int b, int q) { return q < 4 || (q == 4 && b == 0); }
+
 // Second butterfly of a thread in the last step: B - t, so that a thread
 // holds both z_j and z_{L-j} (t = 0: B / 2, its own mirror image).
 template <int Q> __device__ __forceinline__ int fix_b(int t, int n)
@@ -643,7 +663,7 @@ k_rows_fix(const double2 *tw, double2 *Z, SpOut o)
     __shared__ double red[(F::T + 31) / 32];
     pdl_wait();
     pdl_trigger();
-    constexpr int M = F::M, L = F::L, N = F::N, pitch = z_pitch(N);
+    constexpr int M = F::M, N = F::N, pitch = z_pitch(N);
     const int i = blockIdx.x, unit = blockIdx.y, t = threadIdx.x;
     double2 *row = Z + ((int64_t)unit * N + i) * 2 * pitch;
     double2 v[2][8];
@@ -652,7 +672,7 @@ k_rows_fix(const double2 *tw, double2 *Z, SpOut o)
         const int b = fix_b<Q>(t, n);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            const double2 z = row_get(row, pitch, b + q * F::B, M);
+            const double2 z = fix_direct(b, q) ? row[b + q * F::B] : row[pitch + F::B - b + (7 - q) * F::B];
             v[n][q] = DIR ? cswap(z) : z;
         }
     }
@@ -665,10 +685,10 @@ k_rows_fix(const double2 *tw, double2 *Z, SpOut o)
             const int b = fix_b<Q>(t, n);
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-                const int k = b + q * F::B;
-                if (k <= M) row[k] = v[n][q];
-                if (k >= M) row[pitch + L - k] = v[n][q];
-                if (k == 0) row[pitch] = v[n][q];
+                if (fix_direct(b, q)) row[b + q * F::B] = v[n][q];
+                // (elements 0 and M are their own mirror images)
+                if (q >= 4) row[pitch + F::B - b + (7 - q) * F::B] = v[n][q];
+                if (q == 0 && b == 0) row[pitch] = v[n][q];
             }
         }
     } else {
@@ -698,7 +718,7 @@ k_rows_fix(const double2 *tw, double2 *Z, SpOut o)
 // Two columns per block, lanes alternating between them (32-byte sectors).
 template <int Q>
 __global__ void __launch_bounds__(2 * Fix<Q>::T, Q >= 8 ? 512 / (2 * Fix<Q>::T) : 1)
-k_cols_fix(const double2 *tw, const double *f0, const double *f1, double2 *Z, double *colsum)
+k_cols_fix(const double2 *tw, const double2 *twr, const double *f0, const double *f1, double2 *Z, double *colsum)
 {
     using F = Fix<Q>;
     __shared__ __align__(16) double2 s2[2 * sp_line(F::L)];
@@ -718,9 +738,10 @@ k_cols_fix(const double2 *tw, const double *f0, const double *f1, double2 *Z, do
         const int b = fix_b<Q>(t, n);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            const int idx = b + q * F::B;
-            const double2 z = idx <= M ? col[(int64_t)idx * 2 * pitch] : col[(int64_t)(L - idx) * 2 * pitch + m1];
-            v[n][q] = idx <= M ? z : make_double2(sgn * z.x, sgn * z.y);
+            const bool direct = fix_direct(b, q);
+            const double2 z = direct ? col[(b + q * F::B) * 2 * pitch]
+                                     : col[(F::B - b + (7 - q) * F::B) * 2 * pitch + m1];
+            v[n][q] = direct ? z : make_double2(sgn * z.x, sgn * z.y);
         }
     }
     fix_line<Q>(v, s, tw, t);
@@ -731,24 +752,24 @@ k_cols_fix(const double2 *tw, const double *f0, const double *f1, double2 *Z, do
         const int b = fix_b<Q>(t, n);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            const int idx = b + q * F::B;
-            const double g = f[idx <= M ? idx : L - idx];
+            const double g = f[fix_direct(b, q) ? b + q * F::B : F::B - b + (7 - q) * F::B];
             v[n][q] = make_double2(g * v[n][q].y, g * v[n][q].x);
         }
     }
     __syncthreads();   // the last step's reads are done
-    fix_line<Q>(v, s, tw, t);
+    // the reversed plan's factors are the same (8, Q, 8): as a table of their
+    // own they are loaded again instead of being kept in 100 registers
+    fix_line<Q>(v, s, twr, t);
     if (!live) return;
 #pragma unroll
     for (int n = 0; n < 2; n++) {
         const int b = fix_b<Q>(t, n);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-            const int idx = b + q * F::B;
             const double2 z = cswap(v[n][q]), zs = make_double2(sgn * z.x, sgn * z.y);
-            if (idx <= M) col[(int64_t)idx * 2 * pitch] = z;
-            if (idx >= M) col[(int64_t)(L - idx) * 2 * pitch + pitch] = zs;
-            if (idx == 0) col[pitch] = zs;
+            if (fix_direct(b, q)) col[(b + q * F::B) * 2 * pitch] = z;
+            if (q >= 4) col[(F::B - b + (7 - q) * F::B) * 2 * pitch + pitch] = zs;
+            if (q == 0 && b == 0) col[pitch] = zs;
         }
     }
     if (unit == 1 && t == 0)
@@ -762,7 +783,8 @@ static int solve_fix(const OpsView &v, double2 *Z, double *colsum, const SpOut &
     cudaError_t e = launch_after(k_rows_fix<Q, 0>, dim3(N, 2), dim3(T), 0, st, v.tw, Z, o);
     if (e != cudaSuccess) return cuda_check(e, "row transforms launch");
     count_launch();
-    e = launch_after(k_cols_fix<Q>, dim3((N + 1) / 2, 2), dim3(2 * T), 0, st, v.tw, v.f[0], v.f[1], Z, colsum);
+    e = launch_after(k_cols_fix<Q>, dim3((N + 1) / 2, 2), dim3(2 * T), 0, st, v.tw, v.twr, v.f[0], v.f[1], Z,
+                     colsum);
     if (e != cudaSuccess) return cuda_check(e, "column transforms launch");
     count_launch();
     e = launch_after(k_rows_fix<Q, 1>, dim3(N, 2), dim3(T), 0, st, v.tw, Z, o);
@@ -843,8 +865,12 @@ int spectral_solve(const lcb_compute_fields_args *a, const void *ops, cudaStream
     const DftPlan pr = reversed(p);
     int rc = launch_rows_any<0>(N, p, v.tw, Z, o, st);
     if (rc) return rc;
-    rc = any_smem(p.L, 2) <= 220 * 1024 ? launch_cols_any<2>(N, p, pr, v, Z, colsum, st)
-                                        : launch_cols_any<1>(N, p, pr, v, Z, colsum, st);
+    // two columns per block read whole 32-byte sectors, but past L = 1100 two of
+    // their buffers leave room for two blocks per SM only (whole solves with
+    // two columns and with one: L = 768 48 / 52 us, 900 84 / 85, 1152 110 / 107,
+    // 1280 175 / 139)
+    rc = p.L < 1100 ? launch_cols_any<2>(N, p, pr, v, Z, colsum, st)
+                    : launch_cols_any<1>(N, p, pr, v, Z, colsum, st);
     if (rc) return rc;
     return launch_rows_any<1>(N, p, v.tw, Z, o, st);
 }
