@@ -297,7 +297,8 @@ typedef struct lcb_beam_step_args {
 /* One xi step of the beam with every count kept on the device: push layer
  * i-1 (fresh particles get their substep sizes first) followed by the
  * particles that fell from the previous push, compact in order: moved ->
- * drain, fell -> fell_out, lost -> lost; then deposit the layout layer into
+ * drain, fell -> fell_out, lost -> lost (a lost particle that has also fallen
+ * goes into both, as in the reference's masks); then deposit the layout layer into
  * ro0 and ro1, ro1 having been cleared by the push's grid (with three
  * rotating planes it last held the density that the plasma step of layer i
  * has just read).  The deposit only reads the source, so a caller may lay

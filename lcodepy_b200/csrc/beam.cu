@@ -399,7 +399,9 @@ __device__ void compact(const CompactArgs &a, int block, int blocks)
         } else if (f & 4) {
             if (of + pf < a.fell_capacity) soa_store(a.fout, of + pf, v, id, rem);
             else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
-        } else if ((f & 1) && a.lost.id) {
+        }
+        // (a lost particle that has also fallen goes into both buffers)
+        if ((f & 1) && a.lost.id) {
             if (ol + pl < a.lost_capacity) soa_store(a.lost, ol + pl, v, id, rem);
             else if (a.err) atomicOr(a.err, LCB_DEVERR_CAPACITY);
         }
