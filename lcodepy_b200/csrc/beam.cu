@@ -116,11 +116,8 @@ __device__ uint8_t push_particle(int sub, const PushParams &P, const FieldPair &
     }
     while (r > 0) {
         double gm = sqrt(im * im + px * px + py * py + pz * pz);
-        // p / gm: the longitudinal one as a quotient (it is subtracted from 1),
-        // the others by the reciprocal; the same for the rotation's factors
-        double ig = rcp_nr(gm);
-        const double xh = x + dt / 2. * (px * ig);
-        const double yh = y + dt / 2. * (py * ig);
+        const double xh = x + dt / 2. * (px / gm);
+        const double yh = y + dt / 2. * (py / gm);
         const double xih = xi + dt / 2. * (pz / gm - 1);
         if (xih < P.xi_k1) { fell = true; break; }
         if (xh * xh + yh * yh >= P.r_max * P.r_max) {
@@ -174,20 +171,17 @@ __device__ uint8_t push_particle(int sub, const PushParams &P, const FieldPair &
         const double bp = bx * pxm + by * pym + bz * pzm;
         const double g2 = gm * gm - bsq;
         gm = sqrt((g2 + sqrt(g2 * g2 + 4 * bsq + 4 * bp * bp)) / 2.);
-        ig = rcp_nr(gm);
-        const double tx = bx * ig, ty = by * ig, tz = bz * ig;
+        const double tx = bx / gm, ty = by / gm, tz = bz / gm;
         const double tp = 1. + tx * tx + ty * ty + tz * tz;
         const double tmn = 1. - tx * tx - ty * ty - tz * tz;
-        const double itp = rcp_nr(tp), mix = tmn * itp;
-        const double sx = 2. * tx * itp, sy = 2. * ty * itp, sz = 2. * tz * itp;
+        const double sx = 2. * tx / tp, sy = 2. * ty / tp, sz = 2. * tz / tp;
         const double sp = sx * pxm + sy * pym + sz * pzm;
-        px = tx * sp + pxm * mix + pym * sz - pzm * sy + hd * Ex;
-        py = ty * sp + pym * mix + pzm * sx - pxm * sz + hd * Ey;
-        pz = tz * sp + pzm * mix + pxm * sy - pym * sx + hd * Ez;
+        px = tx * sp + pxm * tmn / tp + pym * sz - pzm * sy + hd * Ex;
+        py = ty * sp + pym * tmn / tp + pzm * sx - pxm * sz + hd * Ey;
+        pz = tz * sp + pzm * tmn / tp + pxm * sy - pym * sx + hd * Ez;
         gm = sqrt(im * im + px * px + py * py + pz * pz);
-        ig = rcp_nr(gm);
-        x = xh + dt / 2. * (px * ig);
-        y = yh + dt / 2. * (py * ig);
+        x = xh + dt / 2. * (px / gm);
+        y = yh + dt / 2. * (py / gm);
         xi = xih + dt / 2. * (pz / gm - 1);
         if (x * x + y * y >= P.r_max * P.r_max) { lost = true; r = 0; break; }
         r -= 1;

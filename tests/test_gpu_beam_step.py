@@ -17,6 +17,7 @@ if not torch.cuda.is_available():  # pragma: no cover
 from lcodepy_b200 import _lib  # noqa: E402
 from lcodepy_b200.beam3d import BeamCalculator, BeamParticles, BeamSource  # noqa: E402
 from lcodepy_b200.config import Config  # noqa: E402
+from oracle import oracle as O  # noqa: E402
 
 DEV = torch.device("cuda")
 STATE = ("xi", "x", "y", "px", "py", "pz")
@@ -107,3 +108,47 @@ def test_layer_step_against_its_parts(n, in_place):
         np.testing.assert_array_equal(getattr(bc.lost, name)[:k].cpu().numpy(), p[name].cpu().numpy()[lost])
     if n > 1:
         assert (bc.drain.id[int(moved.sum()):] == -7).all()
+
+
+@pytest.mark.parametrize("n", [3000, 20000])
+def test_push_of_any_mass_against_the_oracle(n):
+    """Both forms of the push against the oracle, a third of the particles
+    without charge over mass (infinitely heavy: they do not move, their
+    momenta grow).  A step of 0.8 layers leaves some in the layer and lets
+    others fall.  As many substeps, gathers and square roots as for any beam:
+    the bound is that of the push's other test."""
+    N, h, dxi, layer = 65, 0.05, 0.05, 9
+    rng = np.random.default_rng(n)
+    p = O.Params(N=N, h=h, dxi=dxi, sub_coeff=1, boundary=0)
+    b = O.Beam(xi=rng.uniform(-layer * dxi, -(layer - 1) * dxi, n), x=rng.normal(0, 0.4, n), y=rng.normal(0, 0.4, n),
+               px=rng.normal(0, 1, n), py=rng.normal(0, 1, n), pz=rng.choice([0.3, 20.0, 1000.0], n),
+               q_m=rng.choice([-1.0, 1 / 1836.0, 0.0], n), q_norm=np.ones(n), id=np.arange(1, n + 1, dtype=np.int64),
+               dt=np.zeros(n), remaining_steps=np.zeros(n, np.int64))
+    X, Y = np.meshgrid(np.arange(N), np.arange(N), indexing="ij")
+    F = [O.Fields(*(0.3 * np.sin(0.2 * (i + 1 + s) * X + 0.1 * Y) for i in range(6)), np.zeros((N, N)))
+         for s in (0, 0.3)]
+    planes = [Planes(torch.stack([torch.tensor(getattr(f, k), device=DEV) for k in
+                                  ("Ex", "Ey", "Ez", "Bx", "By", "Bz", "Phi")])) for f in F]
+    g = {k: torch.tensor(getattr(b, k), device=DEV) for k in STATE + ("q_m", "id", "dt", "remaining_steps")}
+    heavy = b.q_m == 0
+    lost, moved, fell = O.move_beam_layer(p, b, 0, layer, *F, 0.04, 2.0)
+    L, st = _lib.load(), _lib.stream_handle()
+    _lib.check(L.lcb_beam_substepping(n, g["q_m"].data_ptr(), g["pz"].data_ptr(), 2.0, 0.04, g["dt"].data_ptr(),
+                                      g["remaining_steps"].data_ptr(), st), "substepping")
+    flags = torch.zeros(n, dtype=torch.uint8, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    R = h * N / 2
+    _lib.check(L.lcb_beam_move(n, dxi, max(0.9 * R, R - 1), layer - 1, h, N, g["q_m"].data_ptr(), g["dt"].data_ptr(),
+                               C.byref(planes[0].struct), C.byref(planes[1].struct), g["remaining_steps"].data_ptr(),
+                               g["id"].data_ptr(), *(g[k].data_ptr() for k in ("x", "y", "xi", "px", "py", "pz")),
+                               flags.data_ptr(), err.data_ptr(), st), "lcb_beam_move")
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    f = flags.cpu().numpy()
+    assert (heavy & ((f & 2) > 0)).any() and (heavy & ((f & 4) > 0)).any()
+    for bit, ref in ((1, lost), (2, moved), (4, fell)):
+        sel = (f & bit) > 0
+        np.testing.assert_array_equal(g["id"].cpu().numpy()[sel], ref.id)
+        for k in STATE:
+            want = getattr(ref, k)
+            assert np.abs(g[k].cpu().numpy()[sel] - want).max(initial=0) <= 1e-11 * np.abs(want).max(initial=1e-300), k
