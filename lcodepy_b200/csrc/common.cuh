@@ -96,12 +96,17 @@ __device__ __forceinline__ void weights4(double x, double w[5])
     w[4] = b * b * b * b * r24;
 }
 
-// 1 / x and sqrt(x) for normal positive x by Newton's method from the
-// hardware's approximations (about 2^-20): a step of third order for the
-// reciprocal, two coupled second-order steps for the root, within two units
-// in the last place.  Shorter chains than the correctly rounded operations,
-// of which a particle's push has four to five each in sequence (a block of
-// the plasma stage spent 5.4k cycles in it with those, 3.2k with these).
+// 1 / x and sqrt(x) for normal x (the root: positive) by Newton's method from
+// the hardware's approximations (about 2^-20): a step of third order for the
+// reciprocal, two coupled second-order steps for the root.  The last operation
+// is one rounding of a value that is good to 2^-60, so they are within 0.51
+// units in the last place.  Shorter chains than the correctly rounded
+// operations, of which a particle's push has four to five each in sequence.
+// Zeros and infinities give NaN: the plasma's push has none where it gave
+// numbers with the operations themselves (its sums of squares hold a mass, and
+// an overflowed or vanishing gamma - p_z meets an infinity times zero there
+// all the same); the beam's push, where an infinite mass is meaningful, does
+// not use them.
 __device__ __forceinline__ double rcp_nr(double x)
 {
     double r;
