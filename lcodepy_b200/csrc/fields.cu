@@ -1840,8 +1840,11 @@ extern "C" int lcb_field_operators_build(int grid_steps, double h, double subtra
 extern "C" size_t lcb_compute_fields_workspace_bytes(int grid_steps, int precision)
 {
     if (grid_steps < 5) return 0;
-    return precision == LCB_PREC_MIXED ? work_bytes<float>(grid_steps)
-                                       : work_bytes<double>(grid_steps);
+    const size_t dense = precision == LCB_PREC_MIXED ? work_bytes<float>(grid_steps)
+                                                     : work_bytes<double>(grid_steps);
+    // enough for either solver, as LCB_WAVE_KERNEL may ask for the dense one
+    const size_t fast = spectral_grid(grid_steps) ? spectral_work_bytes(grid_steps) : 0;
+    return dense > fast ? dense : fast;
 }
 
 // ---------------------------------------------------------------------------
