@@ -17,33 +17,36 @@
 // and Ey and Bx the odd ones, so Z_k is already a packed line for the second
 // transform: its even part less its odd part, the values of the mirrored
 // nodes, is -Z_{L-k}.  For unit 1 it is +Z_{L-k}.  Nothing is taken apart
-// between the two directions.  The solver's spectral factor 1 / (lam_x +
+// between the two directions.  What a complex transform rounds is relative to
+// the largest of the numbers that it carries, so each field enters multiplied
+// by the power of two that brings its largest right-hand side near one, and
+// leaves divided by it: a small field beside a large one keeps its own
+// precision.  Phi is not a derivative of the currents as Bz and Ez are, and its
+// low modes grow in the solution, so it enters smaller (spectral_solve).  The solver's spectral factor 1 / (lam_x +
 // lam_y + shift) is the same for all the fields of a unit and even along the
 // line, so it multiplies the packed spectrum as it is.
 //
-// The four: right-hand sides, packed; transforms of the rows; transforms of
-// the columns, spectral factor, and back; rows back, with the half/full
-// combinations, the Dirichlet edges and Bz's mean removal.  One FP64 buffer
-// Z[unit][i][s][k] (s = 0: index k, s = 1: index L - k of the line) is
-// transformed in place.  The scratch of a 513 grid is 16.8 MB and stays in
+// The four: right-hand sides and each block's largest of every field; rows
+// scaled, packed and transformed; transforms of the columns, spectral factor,
+// and back; rows back, with the half/full combinations, the Dirichlet edges and
+// Bz's mean removal.  One FP64 buffer Z[unit][i][s][k] is transformed in place
+// (s = 0: index k, s = 1: index L - k of the line; of the right-hand sides s =
+// 0 holds the even fields of node k and s = 1 the odd ones).  The scratch of a 513 grid is 16.8 MB and stays in
 // L2.
 //
 // What bounds it: the inputs and outputs of a 513 grid are 97 MB (15 us at
-// 6.65 TB/s), the transforms 0.2 GFLOP of FP64.  As dense products on the
+// 6.45 TB/s), the transforms 0.2 GFLOP of FP64.  As dense products on the
 // tensor cores (fields.cu, exact int8 slices) the same solve took 187 us in
-// FP64 and 105 us in mixed precision (without Phi), against 54.5 and 50 us
-// with these kernels at first and 50 and 44 us now: 36 slice products per
+// FP64 and 105 us in mixed precision (without Phi), against 50 and 46 us with
+// these kernels (inputs that change from call to call): 36 slice products per
 // multiply-add and N multiply-adds per node and transform cost more than log N
-// FP64 operations on the vector units.  At 129 the solve went from 62.9 to
-// 31.6 us (four launches instead of eleven), at 331, with the kernels for any
-// length, from 83.9 to 47 us.  Of the 50 us (cold, each by itself) the
-// right-hand sides take 15, the rows 10, the columns 17.5 and the rows back 14:
-// latency at 16 warps per SM, the L2's 32-byte sectors in the columns.  The error
-// against 64-bit sums is 6e-16 (dense: 1e-14 FP64, 1e-6 mixed, at 513).
-//
-// Rounding of one field reaches the others of its unit at 2^-53 of the
-// largest of them; the right-hand sides of a unit are differences of the same
-// densities and carry the rounding of those already.
+// FP64 operations on the vector units.  At 129 the solve went from 63 to 32 us
+// (four launches instead of eleven), at 331, with the kernels for any length,
+// from 84 to 52 us.  Finding the scales costs 0.5 to 1.5 us of each kernel of
+// the rows and of the right-hand sides; without them (one rounding size for all
+// the fields of a unit) 385 takes 48.0 us instead of 49.5, 641 139 instead of
+// 141.  The error against 64-bit sums is 6e-16 of each field (dense: 1e-14
+// FP64, 1e-6 mixed, at 513).
 #include <map>
 #include <mutex>
 
@@ -199,10 +202,24 @@ size_t spectral_ops_bytes(int N)
            round256(q.entries * sizeof(double2));
 }
 
-// Z[unit][i][s][k], then the column sums of Bz.
+// Z[unit][i][s][k], then the column sums of Bz, then the blocks' largest
+// exponents and the fields' scales.
 __host__ __device__ constexpr int z_pitch(int N) { return N + 1; }
 static size_t z_bytes(int N) { return round256((size_t)2 * N * 2 * z_pitch(N) * sizeof(double2)); }
-size_t spectral_work_bytes(int N) { return z_bytes(N) + round256((size_t)N * sizeof(double)); }
+static size_t colsum_bytes(int N) { return round256((size_t)N * sizeof(double)); }
+
+// Most blocks of the right-hand sides' kernel: every block of the rows reads
+// what all of them found.  A block has one patch of nodes up to this number of
+// patches (grids up to 760 or so), several above; the loop over them costs 4 us
+// of 57 at 513, which is why it has an instance of its own.
+constexpr int SPR_BLOCKS = 16 * 148;
+
+struct Scales {
+    uint2 part[2][SPR_BLOCKS];   // per unit and block: biased exponents (A.x, B.x | A.y, B.y), 16 bits each
+    double inv[2][4];            // per unit: what A.x, B.x, A.y, B.y are multiplied by on the way out, halved
+};
+
+size_t spectral_work_bytes(int N) { return z_bytes(N) + colsum_bytes(N) + round256(sizeof(Scales)); }
 
 // 4 / h^2 sin^2(k pi / (2 (N - 1)))   (initialization.py:22-24)
 __device__ double sp_lam(int k, int N, double h)
@@ -261,9 +278,12 @@ int spectral_ops_build(int N, double h, double c, void *ops, cudaStream_t st)
 }
 
 // ---------------------------------------------------------------------------
-// Right-hand sides (fields.py:112-230), packed.  A block computes an 8 x 32
-// patch of nodes; the summed half-step densities and the full currents it
-// differentiates are staged with a one-node halo in shared memory.
+// Right-hand sides (fields.py:112-230).  A block computes patches of 8 x 32
+// nodes; the summed half-step densities and the full currents it
+// differentiates are staged with a one-node halo in shared memory.  It leaves
+// the largest exponent of each field among its patches.  Four blocks per SM:
+// the registers of a fifth and sixth hold more of a thread's loads in flight
+// (solve at 513: 50.2 us, 54.0 with 48 registers, 56.1 with 40).
 // ---------------------------------------------------------------------------
 struct SpRhsArgs {
     int N;
@@ -283,65 +303,150 @@ __device__ __forceinline__ double sp_sum(const double *a, int np, int64_t plane,
 
 constexpr int SPR_TY = 8, SPR_TX = 32;
 
-__global__ void __launch_bounds__(SPR_TX * SPR_TY) k_rhs_packed(SpRhsArgs a, double2 *Z)
+// The biased exponents of two values, into a running maximum of 16 bits each
+__device__ __forceinline__ void sp_largest(unsigned &m, double v0, double v1)
+{
+    const unsigned a = (unsigned)__double2hiint(v0) & 0x7ff00000u, b = (unsigned)__double2hiint(v1) & 0x7ff00000u;
+    m = __vmaxu2(m, __byte_perm(a, b, 0x7632) >> 4);
+}
+
+template <bool MANY>
+__global__ void __launch_bounds__(SPR_TX * SPR_TY, 4) k_rhs(SpRhsArgs a, int patches_x, int patches, double2 *Z,
+                                                                Scales *sc)
 {
     pdl_wait();
     pdl_trigger();
     __shared__ double s_ro[SPR_TY + 2][SPR_TX + 2], s_jz[SPR_TY + 2][SPR_TX + 2];
     __shared__ double s_jx[SPR_TY + 2][SPR_TX + 2], s_jy[SPR_TY + 2][SPR_TX + 2];
+    __shared__ unsigned s_w[SPR_TY][4];
     const int N = a.N;
     const int64_t plane = (int64_t)N * N;
-    const int i0 = blockIdx.y * SPR_TY - 1, j0 = blockIdx.x * SPR_TX - 1;
     const int tid = threadIdx.y * SPR_TX + threadIdx.x;
-    for (int e = tid; e < (SPR_TY + 2) * (SPR_TX + 2); e += SPR_TX * SPR_TY) {
-        const int li = e / (SPR_TX + 2), lj = e % (SPR_TX + 2);
-        const int gi = i0 + li, gj = j0 + lj;
-        double ro = 0, jz = 0, jx = 0, jy = 0;
-        if (gi >= 0 && gi < N && gj >= 0 && gj < N) {
-            const int64_t q = (int64_t)gi * N + gj;
-            const double rbf = a.rb_full[q] * a.irb, rbp = a.rb_prev[q] * a.irb;
-            // (full + rho_beam_full + prev + rho_beam_prev) / 2, fields.py:194-197
-            ro = (sp_sum(a.ro_f, a.n_f, plane, q) + rbf + sp_sum(a.ro_p, a.n_p, plane, q) + rbp) / 2;
-            jz = (sp_sum(a.jz_f, a.n_f, plane, q) + rbf + sp_sum(a.jz_p, a.n_p, plane, q) + rbp) / 2;
-            jx = sp_sum(a.jx_f, a.n_f, plane, q);
-            jy = sp_sum(a.jy_f, a.n_f, plane, q);
+    unsigned top[4] = {0, 0, 0, 0};   // (Ey, Ex), (Bx, By), (Bz, Ez), (-, Phi): 16 bits each
+    const int block = MANY ? blockIdx.x : blockIdx.y * gridDim.x + blockIdx.x;
+    for (int patch = block; MANY ? patch < patches : patch == block; patch += MANY ? gridDim.x : 1) {
+        const int i0 = (MANY ? patch / patches_x : blockIdx.y) * SPR_TY - 1;
+        const int j0 = (MANY ? patch % patches_x : blockIdx.x) * SPR_TX - 1;
+        if (MANY) __syncthreads();   // the last patch has been read
+        for (int e = tid; e < (SPR_TY + 2) * (SPR_TX + 2); e += SPR_TX * SPR_TY) {
+            const int li = e / (SPR_TX + 2), lj = e % (SPR_TX + 2);
+            const int gi = i0 + li, gj = j0 + lj;
+            double ro = 0, jz = 0, jx = 0, jy = 0;
+            if (gi >= 0 && gi < N && gj >= 0 && gj < N) {
+                const int64_t q = (int64_t)gi * N + gj;
+                const double rbf = a.rb_full[q] * a.irb, rbp = a.rb_prev[q] * a.irb;
+                // (full + rho_beam_full + prev + rho_beam_prev) / 2, fields.py:194-197
+                ro = (sp_sum(a.ro_f, a.n_f, plane, q) + rbf + sp_sum(a.ro_p, a.n_p, plane, q) + rbp) / 2;
+                jz = (sp_sum(a.jz_f, a.n_f, plane, q) + rbf + sp_sum(a.jz_p, a.n_p, plane, q) + rbp) / 2;
+                jx = sp_sum(a.jx_f, a.n_f, plane, q);
+                jy = sp_sum(a.jy_f, a.n_f, plane, q);
+            }
+            s_ro[li][lj] = ro; s_jz[li][lj] = jz; s_jx[li][lj] = jx; s_jy[li][lj] = jy;
         }
-        s_ro[li][lj] = ro; s_jz[li][lj] = jz; s_jx[li][lj] = jx; s_jy[li][lj] = jy;
+        __syncthreads();
+        const int li = threadIdx.y + 1, lj = threadIdx.x + 1;
+        const int i = i0 + li, j = j0 + lj;
+        if (i >= N || j >= N) continue;
+        const int64_t t = (int64_t)i * N + j;
+        const bool in_x = i >= 1 && i < N - 1, in_y = j >= 1 && j < N - 1, inner = in_x && in_y;
+        double dro_dx = 0, dro_dy = 0, djz_dx = 0, djz_dy = 0, bz = 0, ez = 0, phi = 0;
+        if (inner) {
+            dro_dx = (s_ro[li + 1][lj] - s_ro[li - 1][lj]) * a.i2h;
+            dro_dy = (s_ro[li][lj + 1] - s_ro[li][lj - 1]) * a.i2h;
+            djz_dx = (s_jz[li + 1][lj] - s_jz[li - 1][lj]) * a.i2h;
+            djz_dy = (s_jz[li][lj + 1] - s_jz[li][lj - 1]) * a.i2h;
+            const double djx_dy = s_jx[li][lj + 1] - s_jx[li][lj - 1];
+            const double djy_dx = s_jy[li + 1][lj] - s_jy[li - 1][lj];
+            const double djx_dx = s_jx[li + 1][lj] - s_jx[li - 1][lj];
+            const double djy_dy = s_jy[li][lj + 1] - s_jy[li][lj - 1];
+            bz = -(djx_dy - djy_dx) * a.i2h;
+            ez = -(djx_dx + djy_dy) * a.i2h;
+            if (a.with_phi) phi = sp_sum(a.ro_f, a.n_f, plane, t) - sp_sum(a.jz_f, a.n_f, plane, t);
+        }
+        const double djx_dxi = (sp_sum(a.jx_p, a.n_p, plane, t) - s_jx[li][lj]) * a.idxi;
+        const double djy_dxi = (sp_sum(a.jy_p, a.n_p, plane, t) - s_jy[li][lj]) * a.idxi;
+        // sources that their transforms do not see (the Dirichlet edges) are zero
+        const double ex = in_y ? -(dro_dx - djx_dxi - a.c * a.Ex[t]) : 0.0;
+        const double ey = in_x ? -(dro_dy - djy_dxi - a.c * a.Ey[t]) : 0.0;
+        const double bx = in_x ? +(djz_dy - djy_dxi + a.c * a.Bx[t]) : 0.0;
+        const double by = in_y ? -(djz_dx - djx_dxi - a.c * a.By[t]) : 0.0;
+        const int pitch = z_pitch(N);
+        double2 *z0 = Z + ((int64_t)i * 2) * pitch + j;
+        double2 *z1 = z0 + (int64_t)N * 2 * pitch;
+        z0[0] = make_double2(ey, bx);
+        z0[pitch] = make_double2(ex, by);
+        z1[0] = make_double2(bz, 0.0);
+        z1[pitch] = make_double2(ez, phi);
+        sp_largest(top[0], ey, ex); sp_largest(top[1], bx, by);
+        sp_largest(top[2], bz, ez); sp_largest(top[3], 0.0, phi);
     }
+    // the four words over the warp: half of them stay with each half of the
+    // lanes, then one with each quarter
+    const bool up = threadIdx.x & 16, up2 = threadIdx.x & 8;
+    const unsigned a0 = __vmaxu2(top[up ? 2 : 0], __shfl_xor_sync(0xffffffffu, top[up ? 0 : 2], 16));
+    const unsigned a1 = __vmaxu2(top[up ? 3 : 1], __shfl_xor_sync(0xffffffffu, top[up ? 1 : 3], 16));
+    unsigned m = __vmaxu2(up2 ? a1 : a0, __shfl_xor_sync(0xffffffffu, up2 ? a0 : a1, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) m = __vmaxu2(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 7) == 0) s_w[threadIdx.y][threadIdx.x >> 3] = m;
     __syncthreads();
-    const int li = threadIdx.y + 1, lj = threadIdx.x + 1;
-    const int i = i0 + li, j = j0 + lj;
-    if (i >= N || j >= N) return;
-    const int64_t t = (int64_t)i * N + j;
-    const bool in_x = i >= 1 && i < N - 1, in_y = j >= 1 && j < N - 1, inner = in_x && in_y;
-    double dro_dx = 0, dro_dy = 0, djz_dx = 0, djz_dy = 0, bz = 0, ez = 0, phi = 0;
-    if (inner) {
-        dro_dx = (s_ro[li + 1][lj] - s_ro[li - 1][lj]) * a.i2h;
-        dro_dy = (s_ro[li][lj + 1] - s_ro[li][lj - 1]) * a.i2h;
-        djz_dx = (s_jz[li + 1][lj] - s_jz[li - 1][lj]) * a.i2h;
-        djz_dy = (s_jz[li][lj + 1] - s_jz[li][lj - 1]) * a.i2h;
-        const double djx_dy = s_jx[li][lj + 1] - s_jx[li][lj - 1];
-        const double djy_dx = s_jy[li + 1][lj] - s_jy[li - 1][lj];
-        const double djx_dx = s_jx[li + 1][lj] - s_jx[li - 1][lj];
-        const double djy_dy = s_jy[li][lj + 1] - s_jy[li][lj - 1];
-        bz = -(djx_dy - djy_dx) * a.i2h;
-        ez = -(djx_dx + djy_dy) * a.i2h;
-        if (a.with_phi) phi = sp_sum(a.ro_f, a.n_f, plane, t) - sp_sum(a.jz_f, a.n_f, plane, t);
+    if (tid < 4) {
+        unsigned r = s_w[0][tid];
+#pragma unroll
+        for (int y = 1; y < SPR_TY; y++) r = __vmaxu2(r, s_w[y][tid]);
+        reinterpret_cast<unsigned *>(&sc->part[tid >> 1][block])[tid & 1] = r;
     }
-    const double djx_dxi = (sp_sum(a.jx_p, a.n_p, plane, t) - s_jx[li][lj]) * a.idxi;
-    const double djy_dxi = (sp_sum(a.jy_p, a.n_p, plane, t) - s_jy[li][lj]) * a.idxi;
-    // sources that their transforms do not see (the Dirichlet edges) are zero
-    const double ex = in_y ? -(dro_dx - djx_dxi - a.c * a.Ex[t]) : 0.0;
-    const double ey = in_x ? -(dro_dy - djy_dxi - a.c * a.Ey[t]) : 0.0;
-    const double bx = in_x ? +(djz_dy - djy_dxi + a.c * a.Bx[t]) : 0.0;
-    const double by = in_y ? -(djz_dx - djx_dxi - a.c * a.By[t]) : 0.0;
-    const int pitch = z_pitch(N);
-    double2 *z0 = Z + ((int64_t)i * 2) * pitch + j;
-    double2 *z1 = z0 + (int64_t)N * 2 * pitch;
-    z0[0] = make_double2(ey + ex, bx + by);
-    z0[pitch] = make_double2(ey - ex, bx - by);
-    z1[0] = make_double2(bz + ez, phi);
-    z1[pitch] = make_double2(bz - ez, -phi);
+}
+
+// What the fields of a unit are multiplied by on the way in (A.x, B.x, A.y,
+// B.y), from the blocks' exponents; T threads, `red`: one word pair per warp.
+template <int T>
+__device__ __forceinline__ void sp_scales(Scales *sc, int unit, int blocks, int phi_shift, bool keep, uint2 *red,
+                                          double (&f)[4])
+{
+    uint2 m = make_uint2(0, 0);
+    for (int k0 = threadIdx.x; k0 < blocks; k0 += 8 * T) {
+        uint2 p[8];
+#pragma unroll
+        for (int g = 0; g < 8; g++) p[g] = k0 + g * T < blocks ? sc->part[unit][k0 + g * T] : make_uint2(0, 0);
+#pragma unroll
+        for (int g = 0; g < 8; g++) {
+            m.x = __vmaxu2(m.x, p[g].x);
+            m.y = __vmaxu2(m.y, p[g].y);
+        }
+    }
+    constexpr int W = T < 32 ? T : 32;
+    constexpr unsigned lanes = T < 32 ? (1u << (T & 31)) - 1u : 0xffffffffu;
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+        m.x = __vmaxu2(m.x, __shfl_xor_sync(lanes, m.x, o));
+        m.y = __vmaxu2(m.y, __shfl_xor_sync(lanes, m.y, o));
+    }
+    if (T > 32) {
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < T / 32; w++) {
+            m.x = __vmaxu2(m.x, red[w].x);
+            m.y = __vmaxu2(m.y, red[w].y);
+        }
+    }
+    const unsigned e4[4] = {m.x & 0xffffu, m.x >> 16, m.y & 0xffffu, m.y >> 16};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        // (a field of zeros or subnormal numbers stays as it is)
+        const int e = e4[q] == 0 ? 1023 : min((int)e4[q] + (unit == 1 && q == 3 ? phi_shift : 0), 2045);
+        f[q] = __hiloint2double((2046 - e) << 20, 0);
+        if (keep && threadIdx.x == 0) sc->inv[unit][q] = 0.5 * __hiloint2double(e << 20, 0);
+    }
+}
+
+// Nodes j and L - j of a row's line, packed from the fields of node j.
+__device__ __forceinline__ void sp_pack(double2 A, double2 B, const double (&f)[4], double2 &zp, double2 &zm)
+{
+    const double ax = A.x * f[0], bx = B.x * f[1], ay = A.y * f[2], by = B.y * f[3];
+    zp = make_double2(ax + bx, ay + by);
+    zm = make_double2(ax - bx, ay - by);
 }
 
 // ---------------------------------------------------------------------------
@@ -353,12 +458,21 @@ struct SpOut {
     const double *colsum;        // Bz's column sums, N values
 };
 
+// Half of what the fields of a unit are multiplied by on the way out, by their
+// places (A.x, B.x, A.y, B.y).
+__device__ __forceinline__ void sp_inverse(const Scales *sc, int unit, double (&u)[4])
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++) u[q] = sc->inv[unit][q];
+}
+
 // G nodes j[0 .. G-1] of row i (live ones: j >= 0).  The previous fields of
 // all of them are read before the first store, so that their latencies
 // overlap (a store may alias what is read next, as far as the compiler knows).
 template <int G>
 __device__ __forceinline__ void sp_emit(const SpOut &o, int unit, int N, int i, const int (&j)[G],
-                                        const double2 (&zp)[G], const double2 (&zm)[G], double mean)
+                                        const double2 (&zp)[G], const double2 (&zm)[G], double mean,
+                                        const double (&u)[4])
 {
     const int64_t t0 = (int64_t)i * N;
     const bool edge_x = i == 0 || i == N - 1;
@@ -377,7 +491,8 @@ __device__ __forceinline__ void sp_emit(const SpOut &o, int unit, int N, int i, 
                 if (j[g] < 0) continue;
                 const double a = q < 2 ? zp[g].x : zp[g].y, b = q < 2 ? zm[g].x : zm[g].y;
                 // Ex and By are the odd parts, Ey and Bx the even ones
-                const double v = (q == 0 || q == 3) ? 0.5 * (a - b) : edge_x ? 0.0 : 0.5 * (a + b);
+                const double s = u[q == 0 ? 1 : q == 1 ? 0 : q];
+                const double v = (q == 0 || q == 3) ? s * (a - b) : edge_x ? 0.0 : s * (a + b);
                 if (o.full[F[q]]) o.full[F[q]][t0 + j[g]] = 2 * v - pv[q][g];
                 if (o.half[F[q]]) o.half[F[q]][t0 + j[g]] = v;
             }
@@ -392,9 +507,9 @@ __device__ __forceinline__ void sp_emit(const SpOut &o, int unit, int N, int i, 
         for (int g = 0; g < G; g++) {
             if (j[g] < 0) continue;
             const int64_t t = t0 + j[g];
-            const double ez = edge_x ? 0.0 : 0.5 * (zp[g].x - zm[g].x);
-            const double bz = 0.5 * (zp[g].x + zm[g].x) - mean;
-            const double phi = edge_x ? 0.0 : 0.5 * (zp[g].y - zm[g].y);
+            const double ez = edge_x ? 0.0 : u[1] * (zp[g].x - zm[g].x);
+            const double bz = u[0] * (zp[g].x + zm[g].x) - mean;
+            const double phi = edge_x ? 0.0 : u[3] * (zp[g].y - zm[g].y);
             if (o.full[2]) o.full[2][t] = ez;
             if (o.half[2]) o.half[2][t] = (ez + pe[g]) / 2;
             if (o.full[5]) o.full[5][t] = bz;
@@ -505,18 +620,29 @@ constexpr int SP_ANY_THREADS = 128;
 // DIR 1: back to the nodes, and out.
 template <int DIR>
 __global__ void __launch_bounds__(SP_ANY_THREADS)
-k_rows_any(int N, const __grid_constant__ DftPlan p, const double2 *tw, double2 *Z, SpOut o)
+k_rows_any(int N, const __grid_constant__ DftPlan p, const double2 *tw, double2 *Z, SpOut o, Scales *sc, int blocks,
+           int phi_shift)
 {
     extern __shared__ __align__(16) double2 line[];
     __shared__ double red[SP_ANY_THREADS / 32];
+    __shared__ uint2 red2[SP_ANY_THREADS / 32];
     pdl_wait();
     pdl_trigger();
     const int M = N - 1, L = p.L, pitch = z_pitch(N), i = blockIdx.x, unit = blockIdx.y;
     double2 *row = Z + ((int64_t)unit * N + i) * 2 * pitch;
     double2 *a = line, *b = line + sp_line(L);
-    for (int idx = threadIdx.x; idx < L; idx += SP_ANY_THREADS) {
-        const double2 z = row_get(row, pitch, idx, M);
-        a[sp_pad(idx)] = DIR ? cswap(z) : z;
+    if (DIR == 0) {
+        double f[4];
+        sp_scales<SP_ANY_THREADS>(sc, unit, blocks, phi_shift, i == 0, red2, f);
+        for (int idx = threadIdx.x; idx <= M; idx += SP_ANY_THREADS) {
+            double2 zp, zm;
+            sp_pack(row[idx], row[pitch + idx], f, zp, zm);
+            a[sp_pad(idx)] = zp;
+            if (idx > 0 && idx < M) a[sp_pad(L - idx)] = zm;
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < L; idx += SP_ANY_THREADS)
+            a[sp_pad(idx)] = cswap(row_get(row, pitch, idx, M));
     }
     __syncthreads();
     a = any_line(p, tw, a, b, threadIdx.x, SP_ANY_THREADS);
@@ -526,7 +652,9 @@ k_rows_any(int N, const __grid_constant__ DftPlan p, const double2 *tw, double2 
             row[pitch + k] = a[sp_pad(k == 0 ? 0 : L - k)];
         }
     } else {
-        const double mean = unit == 1 ? sp_total(o.colsum, N, red) / ((double)N * N) : 0.0;
+        double u[4];
+        sp_inverse(sc, unit, u);
+        const double mean = unit == 1 ? sp_total(o.colsum, N, red) / ((double)N * N) * (2 * u[0]) : 0.0;
         for (int j0 = threadIdx.x; j0 <= M; j0 += 4 * SP_ANY_THREADS) {
             int j[4];
             double2 zp[4], zm[4];
@@ -537,7 +665,7 @@ k_rows_any(int N, const __grid_constant__ DftPlan p, const double2 *tw, double2 
                 zp[g] = cswap(a[sp_pad(jj <= M ? jj : 0)]);
                 zm[g] = cswap(a[sp_pad(jj == 0 || jj > M ? 0 : L - jj)]);
             }
-            sp_emit(o, unit, N, i, j, zp, zm, mean);
+            sp_emit(o, unit, N, i, j, zp, zm, mean, u);
         }
     }
 }
@@ -656,28 +784,57 @@ __device__ __forceinline__ void fix_line(double2 (&v)[2][8], double2 *s, const d
 
 template <int Q, int DIR>
 __global__ void __launch_bounds__(Fix<Q>::T, Q >= 8 ? 512 / Fix<Q>::T : 1)
-k_rows_fix(const double2 *tw, double2 *Z, SpOut o)
+k_rows_fix(const double2 *tw, double2 *Z, SpOut o, Scales *sc, int blocks,
+           int phi_shift)
 {
     using F = Fix<Q>;
     __shared__ __align__(16) double2 s[sp_line(F::L)];
     __shared__ double red[(F::T + 31) / 32];
+    __shared__ uint2 red2[(F::T + 31) / 32];
     pdl_wait();
     pdl_trigger();
     constexpr int M = F::M, N = F::N, pitch = z_pitch(N);
     const int i = blockIdx.x, unit = blockIdx.y, t = threadIdx.x;
     double2 *row = Z + ((int64_t)unit * N + i) * 2 * pitch;
     double2 v[2][8];
+    double u[4], mean = 0;
+    if (DIR == 0) {
+        // the fields of nodes j = b + q B, which are packed into elements j and
+        // L - j = (B - b) + (7 - q) B: a thread's own, as above
+        double2 A[2][4], B[2][4], AM, BM;
 #pragma unroll
-    for (int n = 0; n < 2; n++) {
-        const int b = fix_b<Q>(t, n);
+        for (int n = 0; n < 2; n++)
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const double2 z = fix_direct(b, q) ? row[b + q * F::B] : row[pitch + F::B - b + (7 - q) * F::B];
-            v[n][q] = DIR ? cswap(z) : z;
+            for (int q = 0; q < 4; q++) {
+                const int j = fix_b<Q>(t, n) + q * F::B;
+                A[n][q] = row[j];
+                B[n][q] = row[pitch + j];
+            }
+        AM = BM = make_double2(0.0, 0.0);
+        if (t == 0) { AM = row[M]; BM = row[pitch + M]; }
+        sp_scales<F::T>(sc, unit, blocks, phi_shift, i == 0, red2, u);
+        double2 m[2][4], zM, mM;
+        sp_pack(AM, BM, u, zM, mM);
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) sp_pack(A[n][q], B[n][q], u, v[n][q], m[n][q]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            v[1][7 - q] = t > 0 ? m[0][q] : m[1][q];
+            v[0][7 - q] = t > 0 ? m[1][q] : q < 3 ? m[0][q < 3 ? q + 1 : 0] : zM;
         }
+    } else {
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+            const int b = fix_b<Q>(t, n);
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                v[n][q] = cswap(fix_direct(b, q) ? row[b + q * F::B] : row[pitch + F::B - b + (7 - q) * F::B]);
+        }
+        sp_inverse(sc, unit, u);
+        if (unit == 1) mean = sp_total(o.colsum, N, red) / ((double)N * N) * (2 * u[0]);
     }
-    double mean = 0;
-    if (DIR == 1 && unit == 1) mean = sp_total(o.colsum, N, red) / ((double)N * N);
     fix_line<Q>(v, s, tw, t);
     if (DIR == 0) {
 #pragma unroll
@@ -705,12 +862,12 @@ k_rows_fix(const double2 *tw, double2 *Z, SpOut o)
                 zp[q] = cswap(v[n][q]);
                 zm[q] = cswap(t > 0 ? v[1 - n][7 - q] : n == 0 ? v[0][(8 - q) & 7] : v[1][7 - q]);
             }
-            sp_emit(o, unit, N, i, j, zp, zm, mean);
+            sp_emit(o, unit, N, i, j, zp, zm, mean, u);
         }
         if (t == 0) {
             const int j[1] = {M};
             const double2 z[1] = {cswap(v[0][4])};
-            sp_emit(o, unit, N, i, j, z, z, mean);
+            sp_emit(o, unit, N, i, j, z, z, mean, u);
         }
     }
 }
@@ -777,17 +934,18 @@ k_cols_fix(const double2 *tw, const double2 *twr, const double *f0, const double
 }
 
 template <int Q>
-static int solve_fix(const OpsView &v, double2 *Z, double *colsum, const SpOut &o, cudaStream_t st)
+static int solve_fix(const OpsView &v, double2 *Z, double *colsum, const SpOut &o, Scales *sc, int blocks,
+                     int phi_shift, cudaStream_t st)
 {
     constexpr int N = Fix<Q>::N, T = Fix<Q>::T;
-    cudaError_t e = launch_after(k_rows_fix<Q, 0>, dim3(N, 2), dim3(T), 0, st, v.tw, Z, o);
+    cudaError_t e = launch_after(k_rows_fix<Q, 0>, dim3(N, 2), dim3(T), 0, st, v.tw, Z, o, sc, blocks, phi_shift);
     if (e != cudaSuccess) return cuda_check(e, "row transforms launch");
     count_launch();
     e = launch_after(k_cols_fix<Q>, dim3((N + 1) / 2, 2), dim3(2 * T), 0, st, v.tw, v.twr, v.f[0], v.f[1], Z,
                      colsum);
     if (e != cudaSuccess) return cuda_check(e, "column transforms launch");
     count_launch();
-    e = launch_after(k_rows_fix<Q, 1>, dim3(N, 2), dim3(T), 0, st, v.tw, Z, o);
+    e = launch_after(k_rows_fix<Q, 1>, dim3(N, 2), dim3(T), 0, st, v.tw, Z, o, sc, blocks, phi_shift);
     if (e != cudaSuccess) return cuda_check(e, "row transforms back launch");
     count_launch();
     return LCB_OK;
@@ -809,12 +967,14 @@ static int launch_cols_any(int N, const DftPlan &p, const DftPlan &pr, const Ops
 }
 
 template <int DIR>
-static int launch_rows_any(int N, const DftPlan &p, const double2 *tw, double2 *Z, const SpOut &o, cudaStream_t st)
+static int launch_rows_any(int N, const DftPlan &p, const double2 *tw, double2 *Z, const SpOut &o, Scales *sc,
+                           int blocks, int phi_shift, cudaStream_t st)
 {
     static std::atomic<unsigned long long> attr{0};
     cudaError_t e = ensure_smem(k_rows_any<DIR>, 224 * 1024, attr);
     if (e != cudaSuccess) return cuda_check(e, "row transforms smem attribute");
-    e = launch_after(k_rows_any<DIR>, dim3(N, 2), dim3(SP_ANY_THREADS), any_smem(p.L, 1), st, N, p, tw, Z, o);
+    e = launch_after(k_rows_any<DIR>, dim3(N, 2), dim3(SP_ANY_THREADS), any_smem(p.L, 1), st, N, p, tw, Z, o,
+                     sc, blocks, phi_shift);
     if (e != cudaSuccess) return cuda_check(e, "row transforms launch");
     count_launch();
     return LCB_OK;
@@ -827,7 +987,9 @@ int spectral_solve(const lcb_compute_fields_args *a, const void *ops, cudaStream
     LCB_REQUIRE(plan_of(N, p), "grid_steps %d has no fast transform", N);
     const OpsView v = ops_view(ops, N, p);
     double2 *Z = static_cast<double2 *>(a->workspace);
-    double *colsum = reinterpret_cast<double *>(static_cast<char *>(a->workspace) + z_bytes(N));
+    char *behind = static_cast<char *>(a->workspace) + z_bytes(N);
+    double *colsum = reinterpret_cast<double *>(behind);
+    Scales *sc = reinterpret_cast<Scales *>(behind + colsum_bytes(N));
 
     SpRhsArgs r;
     r.N = N;
@@ -844,10 +1006,22 @@ int spectral_solve(const lcb_compute_fields_args *a, const void *ops, cudaStream
     r.Ex = a->fields.f[0]; r.Ey = a->fields.f[1];
     r.Bx = a->fields.f[3]; r.By = a->fields.f[4];
     r.with_phi = (a->out_half.f[6] || a->out_full.f[6]) ? 1 : 0;
-    cudaError_t e = launch_after(k_rhs_packed, dim3((N + SPR_TX - 1) / SPR_TX, (N + SPR_TY - 1) / SPR_TY),
-                                 dim3(SPR_TX, SPR_TY), 0, st, r, Z);
+    const int patches_x = (N + SPR_TX - 1) / SPR_TX, patches_y = (N + SPR_TY - 1) / SPR_TY;
+    const int patches = patches_x * patches_y, rounds = (patches + SPR_BLOCKS - 1) / SPR_BLOCKS;
+    const int blocks = (patches + rounds - 1) / rounds;
+    const dim3 threads(SPR_TX, SPR_TY);
+    cudaError_t e = rounds == 1
+        ? launch_after(k_rhs<false>, dim3(patches_x, patches_y), threads, 0, st, r, patches_x, patches, Z, sc)
+        : launch_after(k_rhs<true>, dim3(blocks), threads, 0, st, r, patches_x, patches, Z, sc);
     if (e != cudaSuccess) return cuda_check(e, "rhs launch");
     count_launch();
+
+    // The smallest Laplacian eigenvalue lets Phi's solution reach 0.074 W^2 of
+    // its right-hand side, W the grid's width, where Bz's and Ez's stay near one
+    // times theirs at the plasma's wave numbers: half of that factor (in powers
+    // of two) in either direction.
+    const double grow = 0.27 * (N - 1) * a->h;
+    const int phi_shift = grow > 1 ? (int)lround(fmin(log2(grow), 40.0)) : 0;
 
     SpOut o;
     for (int f = 0; f < 7; f++) {
@@ -857,13 +1031,13 @@ int spectral_solve(const lcb_compute_fields_args *a, const void *ops, cudaStream
     }
     o.colsum = colsum;
     switch (fixed_q(p.L)) {
-    case 2: return solve_fix<2>(v, Z, colsum, o, st);
-    case 4: return solve_fix<4>(v, Z, colsum, o, st);
-    case 8: return solve_fix<8>(v, Z, colsum, o, st);
-    case 16: return solve_fix<16>(v, Z, colsum, o, st);
+    case 2: return solve_fix<2>(v, Z, colsum, o, sc, blocks, phi_shift, st);
+    case 4: return solve_fix<4>(v, Z, colsum, o, sc, blocks, phi_shift, st);
+    case 8: return solve_fix<8>(v, Z, colsum, o, sc, blocks, phi_shift, st);
+    case 16: return solve_fix<16>(v, Z, colsum, o, sc, blocks, phi_shift, st);
     }
     const DftPlan pr = reversed(p);
-    int rc = launch_rows_any<0>(N, p, v.tw, Z, o, st);
+    int rc = launch_rows_any<0>(N, p, v.tw, Z, o, sc, blocks, phi_shift, st);
     if (rc) return rc;
     // two columns per block read whole 32-byte sectors, but past L = 1100 two of
     // their buffers leave room for two blocks per SM only (whole solves with
@@ -872,7 +1046,7 @@ int spectral_solve(const lcb_compute_fields_args *a, const void *ops, cudaStream
     rc = p.L < 1100 ? launch_cols_any<2>(N, p, pr, v, Z, colsum, st)
                     : launch_cols_any<1>(N, p, pr, v, Z, colsum, st);
     if (rc) return rc;
-    return launch_rows_any<1>(N, p, v.tw, Z, o, st);
+    return launch_rows_any<1>(N, p, v.tw, Z, o, sc, blocks, phi_shift, st);
 }
 
 }  // namespace lcb
