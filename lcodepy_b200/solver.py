@@ -184,13 +184,18 @@ class Plane2d3vPlasmaSolver:
             if self.n_sorts == 2:
                 s.q[n:] = -q_t
                 s.m[n:] = self.config.getfloat("ion-mass") * m_t
-        # background charge: minus the deposited initial electrons
-        # (initialization.py:351-356)
-        tmp = self.currents[1]
-        self._deposit(st, tmp, with_background=False, n_sorts=1)
-        self.ro_initial.copy_(-tmp.ro[0])
         for f in self.fields + self.half:
             f.buf.zero_()
+        # background charge: minus the deposited initial electrons
+        # (initialization.py:351-356), by the kernel that deposits them in the
+        # xi loop: a difference of two kernels' roundings, small but the same
+        # at every node, would act as a charge of the whole plasma
+        tmp = self.currents[1]
+        if self.fused and max(np.abs(x_init).max(), np.abs(y_init).max()) < self.boundary:
+            self._move_deposit(self.fields[0], st, self.states[1], tmp, True)
+        else:
+            self._deposit(st, tmp, with_background=False, n_sorts=1)
+        self.ro_initial.copy_(-tmp.ro[0])
         for c in self.currents:
             c.buf.zero_()
         self.err.zero_()

@@ -106,3 +106,26 @@ def test_stage_drops_a_particle_that_is_not_a_number(precision):
     torch.cuda.synchronize()
     assert int(ps.err.item()) & _lib.DEVERR_PLASMA_STENCIL
     assert np.isfinite(out.buf.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("N,ppc", [(129, 1), (129, 4), (129, 9)])
+def test_background_cancels_the_electrons_at_rest(N, ppc):
+    """Electrons that have not moved, deposited by the fused stage, against
+    the background charge: what is left is the rounding of single nodes (some
+    1.5 of 2^-53 rms), whose mean over n nodes is 1.5 / sqrt(n) of it, and no
+    common part."""
+    h = 0.05
+    cfg = Config({'geometry': '3d', 'window-width': (N + 0.5) * h / 2, 'transverse-step': h, 'xi-step': h,
+                  'window-length': 1.0, 'ion-model': 'background', 'plasma-particles-per-cell': ppc,
+                  'precision': 'fp64', 'print-every': 0})
+    cfg._adjust_config_values_3d()
+    ps = Plane2d3vPlasmaSolver(cfg, DEV)
+    ps.init_state(0.0)
+    prev, full = ps.states
+    assert all(float(getattr(s, k).abs().max()) == 0 for s in (prev, full) for k in ("x_offt", "y_offt", "px", "py", "pz"))
+    out = CurrentSet(N, DEV)
+    ps._move_deposit(ps.fields[0], prev, full, out, True)
+    left = (out.buf[0][0] + ps.ro_initial).cpu().numpy()[24:-24, 24:-24]
+    np.testing.assert_array_equal(out.buf[0][1].cpu().numpy(), ps.ro_initial.cpu().numpy())
+    assert abs(left.mean()) <= 4 * 1.5 * 2.0 ** -53 / left.size ** 0.5
+    assert (left ** 2).mean() ** 0.5 <= 2.5 * 2.0 ** -53
