@@ -265,15 +265,8 @@ __device__ __forceinline__ void soa_store(const lcb_beam_soa &s, int64_t i, cons
 }
 
 template <int G>
-__global__ void __launch_bounds__(128) k_beam_push_stage(StepArgs a)
+__device__ __forceinline__ void push_stage(const StepArgs &a, int64_t total)
 {
-    pdl_wait();
-    pdl_trigger();
-    if (a.fell_out_count && blockIdx.x == 0 && threadIdx.x == 0) *a.fell_out_count = 0;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < a.clear_n;
-         t += (int64_t)gridDim.x * blockDim.x)
-        a.clear[t] = 0.0;
-    const int64_t total = a.n_fresh + *a.fell_in_count;
     const int sub = threadIdx.x % G;
     for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G; t < total;
          t += (int64_t)gridDim.x * blockDim.x / G) {
@@ -300,6 +293,25 @@ __global__ void __launch_bounds__(128) k_beam_push_stage(StepArgs a)
     }
 }
 
+// The grid is sized by the fresh particles; how many have fallen is known here
+// only.  Groups take what the grid can hold of them twice over, which is all of
+// a layer whose particles are mostly fresh; more than that go one to a thread
+// (a layer step behind the beam, 50,000 fallen particles and none fresh: 54 us,
+// with groups and one compacting block 372; all in single threads and one block
+// of 1024, 207).  GROUPS false: more fresh particles than groups take.
+template <bool GROUPS>
+__global__ void __launch_bounds__(128) k_beam_push_stage(StepArgs a)
+{
+    pdl_wait();
+    pdl_trigger();
+    if (a.fell_out_count && blockIdx.x == 0 && threadIdx.x == 0) *a.fell_out_count = 0;
+    const int64_t threads = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < a.clear_n; t += threads) a.clear[t] = 0.0;
+    const int64_t total = a.n_fresh + *a.fell_in_count;
+    if (GROUPS && total <= BEAM_GROUP_MAX && total * BEAM_GROUP <= 2 * threads) push_stage<BEAM_GROUP>(a, total);
+    else push_stage<1>(a, total);
+}
+
 struct CompactArgs {
     lcb_beam_soa stage, drain, fout, lost;
     const uint8_t *flags;
@@ -315,12 +327,14 @@ struct CompactArgs {
 // where a tile's particles go by counting the flags before it itself (a byte
 // per particle, from L2), so that the blocks do not wait for one another.
 // The counters may only move once every block has read them: the blocks check
-// out at fell_out_count, which the push has zeroed, and the last one writes
-// all three.  The grid's other blocks lay out the next layer meanwhile (that
+// out in the upper bits of fell_out_count (zeroed by the push, or the count of
+// the fallen itself where that is updated in place), and the last one writes all
+// three.  The grid's other blocks lay out the next layer meanwhile (that
 // reads only the source, and the push's grid has cleared ro1).
 // For a layer of 8,300 particles one block over all chunks took 34 us and the
 // layout another 9 after it.
 constexpr int CMP_THREADS = 256, CMP_WARPS = CMP_THREADS / 32;
+constexpr int CMP_CHECK_OUT = 40;   // a count is below 2^40
 
 struct FlagCounts { int moved, fell, lost; };
 
@@ -368,7 +382,7 @@ __device__ void compact(const CompactArgs &a, int block, int blocks)
     __shared__ int red[CMP_WARPS][3], wsum[CMP_WARPS][3];
     __shared__ bool last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int64_t total = a.n_fresh + *a.fell_in_count;
+    int64_t total = a.n_fresh + (*a.fell_in_count & ((int64_t(1) << CMP_CHECK_OUT) - 1));
     if (total > a.stage_capacity) total = a.stage_capacity;
     const int64_t drain0 = *a.drain_count, lost0 = a.lost_count ? *a.lost_count : 0;
     int64_t om = drain0, of = 0, ol = lost0, counted = 0;   // places of the tile's first ones
@@ -403,9 +417,8 @@ __device__ void compact(const CompactArgs &a, int block, int blocks)
     __syncthreads();   // every thread has read the counters
     if (tid == 0) {
         __threadfence();
-        last = blocks == 1 ||
-               atomicAdd(reinterpret_cast<unsigned long long *>(a.fell_out_count), 1ull) ==
-               (unsigned long long)(blocks - 1);
+        last = atomicAdd(reinterpret_cast<unsigned long long *>(a.fell_out_count), 1ull << CMP_CHECK_OUT) >>
+               CMP_CHECK_OUT == (unsigned long long)(blocks - 1);
     }
     __syncthreads();
     if (!last) return;
@@ -537,15 +550,13 @@ extern "C" int lcb_beam_step(const lcb_beam_step_args *a, void *stream)
     }
     s.clear = a->ro1;
     s.clear_n = (int64_t)N * N;
-    // (one block compacts where the counter of the fallen is updated in place)
-    const bool in_place = a->fell_out_count == a->fell_in_count;
-    s.fell_out_count = in_place ? nullptr : a->fell_out_count;
+    s.fell_out_count = a->fell_out_count == a->fell_in_count ? nullptr : a->fell_out_count;
     s.err = a->err;
     // at least two blocks per SM, for the plane and for particles that fell
     // (their number is on the device)
     const bool group = s.n_fresh <= BEAM_GROUP_MAX;
     const int pg = grid_for(group ? s.n_fresh * BEAM_GROUP : s.n_fresh, 128), most = 2 * sm_count();
-    cudaError_t e = launch_after(group ? k_beam_push_stage<BEAM_GROUP> : k_beam_push_stage<1>,
+    cudaError_t e = launch_after(group ? k_beam_push_stage<true> : k_beam_push_stage<false>,
                                  dim3(pg > most ? pg : most), dim3(128), 0, st, s);
     if (e != cudaSuccess) return cuda_check(e, "beam push launch");
     count_launch();
@@ -563,13 +574,14 @@ extern "C" int lcb_beam_step(const lcb_beam_step_args *a, void *stream)
     const LayoutArgs l = {n, N, a->h, a->xi_step, -a->xi_step * (double)a->layout_idx,
                           a->source.x + o, a->source.y + o, a->source.xi + o, a->source.q_norm + o,
                           a->ro0, a->ro1, a->err};
-    // one block per tile of fresh particles and one for those that fell, up to
-    // two per SM; as many again at most for the layout
+    // blocks for every tile that the staging buffer can hold, up to two per SM
+    // (those without a tile only check out: the number of fallen particles is
+    // on the device); as many again at most for the layout
     auto blocks = [&](int64_t threads) {
         const int64_t b = (threads + CMP_THREADS - 1) / CMP_THREADS;
         return (int)(b < most ? b : most);
     };
-    const int nc = in_place ? 1 : blocks(c.n_fresh + CMP_THREADS);
+    const int nc = a->stage_capacity > 0 ? blocks(a->stage_capacity) : 1;
     e = launch_after(k_beam_compact_layout, dim3(nc + blocks(n * BEAM_GROUP)), dim3(CMP_THREADS), 0, st, c, l, nc);
     if (e != cudaSuccess) return cuda_check(e, "beam compaction launch");
     count_launch();

@@ -1,8 +1,9 @@
 """One layer step of the beam against its parts: the push by lcb_beam_move and
 the ordered selection of moved, fallen and lost particles by boolean masks, at
-the edges of the compaction's tiles (256 particles), in both forms of the push
-(a group of lanes per particle up to 16384, a thread each above) and with the
-fallen particles' counter updated in place."""
+the edges of the compaction's tiles (256 particles), with fresh and fallen
+particles and either alone, in both forms of the push (a group of lanes per
+particle up to 16384, a thread each above) and with the fallen particles'
+counter updated in place.  Both forms of the push against the oracle."""
 import ctypes as C
 
 import numpy as np
@@ -49,9 +50,12 @@ def _beam(n, layer, dxi, g):
     return b
 
 
-@pytest.mark.parametrize("n,in_place", [(1, False), (255, False), (256, False), (257, False), (5000, False),
-                                        (5000, True), (20000, False)])
-def test_layer_step_against_its_parts(n, in_place):
+@pytest.mark.parametrize("fresh,fallen,in_place", [
+    (1, 0, False), (255, 0, False), (256, 0, False), (257, 0, False), (5000, 0, False), (5000, 0, True),
+    (20000, 0, False), (0, 1, False), (255, 2, False), (300, 4000, False), (300, 4000, True), (0, 9000, True),
+    (200, 20000, False), (0, 80000, True)])
+def test_layer_step_against_its_parts(fresh, fallen, in_place):
+    n = fresh + fallen
     L = _lib.load()
     N, dxi = 65, 0.05
     cfg = Config({'geometry': '3d', 'window-width': 1.63, 'transverse-step': 0.05, 'window-length': 1.0,
@@ -65,18 +69,21 @@ def test_layer_step_against_its_parts(n, in_place):
     F = [Planes((torch.rand(7, N, N, generator=g, device=DEV, dtype=torch.float64) - 0.5) * 0.4) for _ in range(2)]
     bc = BeamCalculator(cfg, DEV)
     bc.start_time_step(BeamSource(cfg, b, DEV))
+    dt, rs = torch.zeros_like(b.xi), torch.zeros_like(b.id)
+    if fallen:   # two substeps of half a time step left
+        dt[fresh:], rs[fresh:] = 0.5, 2
+        b.dt, b.remaining_steps = dt.clone(), rs.clone()
+        for k in b._all():
+            getattr(bc.fell[0], k)[:fallen] = getattr(b, k)[fresh:]
+        bc.counts[0] = fallen
+    a = bc._args(layer + 1, (0, 0), (0, fresh), F[0], F[1])
     if in_place:
-        bc.counts = torch.zeros_like(bc.counts)
-        a = bc._args(layer + 1, (0, 0), (0, n), F[0], F[1])
         a.fell_out_count = a.fell_in_count
-    else:
-        a = bc._args(layer + 1, (0, 0), (0, n), F[0], F[1])
     bc.drain.id[:] = -7
     _lib.check(L.lcb_beam_step(C.byref(a), _lib.stream_handle()), "lcb_beam_step")
 
-    dt, rs = torch.zeros_like(b.xi), torch.zeros_like(b.id)
     st = _lib.stream_handle()
-    _lib.check(L.lcb_beam_substepping(n, b.q_m.data_ptr(), b.pz.data_ptr(), 2.0, 1.0, dt.data_ptr(), rs.data_ptr(),
+    _lib.check(L.lcb_beam_substepping(fresh, b.q_m.data_ptr(), b.pz.data_ptr(), 2.0, 1.0, dt.data_ptr(), rs.data_ptr(),
                                       st), "substepping")
     p = {k: getattr(b, k).clone() for k in STATE}
     ids = b.id.clone()
