@@ -402,13 +402,17 @@ static size_t deposit_smem_bytes()
 // their weights and values in shared memory), and their stencils summed in
 // registers, a lane taking four cells along x and one quantity, before the
 // sums go to HBM: about 16 additions per particle instead of 100 in shared
-// memory.  Particles whose stencil leaves a window use global memory.
+// memory (mixed precision with one particle per cell: in shared memory all the
+// same, see Stage).  Particles whose stencil leaves a window use global memory.
 // FP64 (FT = double): FP64 window, weights and sums.  Mixed precision
 // (FT = float): coordinates and momenta stay FP64; the gather reads an FP32
-// copy of the field window with FP32 weights (the mixed form's fields carry
-// FP32 accuracy); the deposit keeps FP64 weights, scales each particle's four
+// copy of the field window with FP32 weights; the deposit keeps FP64 weights, scales each particle's four
 // values by 2^32 / h^2 once, and rounds every contribution to an integer with
-// one FMA against FIX_MAGIC, so that the sums are exact.
+// one FMA against FIX_MAGIC, so that the sums are exact.  FP64 sums round as
+// they are added, in an order that the atomics decide: they repeat to their last
+// bits only, a node's density to 1.0 of 2^-53 rms (0.7 with exact block sums of
+// terms in units of 2^-56, which leave currents much smaller than the density
+// less exact, and whose price for the cells in registers is 101 -> 125 us).
 //
 // What bounds it: latency, at the 16 warps per SM that the push's registers
 // leave.  Adding every contribution to a shared window with 32-bit integer
@@ -586,15 +590,35 @@ template <typename FT> struct StageAcc;
 template <> struct StageAcc<float> { typedef fix_t type; };
 template <> struct StageAcc<double> { typedef double type; };
 
+// t = FIX_MAGIC + n, |n| < 2^41, into a sum of shared memory: its low 20 bits to
+// an unsigned word, the rest to a signed one (32-bit integer atomics are native
+// there, 64-bit ones are not).  Of a block's 512 particles neither word overflows.
+__device__ __forceinline__ void shared_fix_add(unsigned *lo, int *hi, double t)
+{
+    const unsigned w0 = (unsigned)__double2loint(t);
+    const unsigned w1 = (unsigned)(__double2hiint(t) - 0x43380000);   // (FIX_MAGIC's low word is zero)
+    atomicAdd(lo, w0 & 0xFFFFFu);
+    atomicAdd(hi, (int)__funnelshift_r(w0, w1, 20));
+}
+
 // Shape of a block of the fused stage: TI x TJ lattice particles, two per
-// thread; a window of WX x WY nodes around them.
-template <typename FT, int WX_, int WY_> struct Stage {
+// thread; a window of WX x WY nodes around them.  SHARED: the deposit adds to
+// node sums in shared memory (mixed precision), else by cells in registers.
+// With one particle per cell along an axis a lane would clear, walk and send 40
+// sums for four particles: a mixed stage at 641 takes 80 us by cells, 65 us
+// with the sums in shared memory (75 us with three blocks per SM and 80
+// registers); at 321 32.3 and 28.5, at 91 19.5 and 18.  With four particles per
+// cell the cells win: 105 us against 93 at 513; they also do where a tile's
+// particles meet in few cells (all in one: 92 us against 160 at 513, one per
+// cell).  FP64 has no exact sums of two words, and stays with the cells.
+template <typename FT, int WX_, int WY_, bool SHARED_ = false> struct Stage {
+    static constexpr bool SHARED = SHARED_;
     static constexpr int TI = 16, TJ = 32, WX = WX_, WY = WY_;
     static constexpr int NP = TI * TJ, THREADS = NP / 2, WARPS = THREADS / 32;
     static constexpr int WSZ = WX * WY;
     static constexpr int CX = WX - 4, CY = WY - 4, NC = CX * CY;   // cells of the window
     // cells along x that one lane of the deposit sums (4: 107 us a production
-    // FP64 stage, 3: 109, 5: 111; with another record layout 4: 114, 1: 129)
+    // FP64 stage, 3: 109, 5: 111)
     static constexpr int XU = 4;
     // a particle's record for the deposit: five weights along x, five along
     // y, four values; the cells' columns a record apart (neighbouring lanes
@@ -603,8 +627,8 @@ template <typename FT, int WX_, int WY_> struct Stage {
     static constexpr int RECORD = 14, SLOTS = NP + CY;
     static constexpr size_t field_bytes = (size_t)WSZ * FieldWin<FT>::bytes_per_cell;
     static constexpr size_t rec_bytes = (size_t)SLOTS * RECORD * sizeof(double);
-    static constexpr size_t main_bytes = field_bytes > rec_bytes ? field_bytes : rec_bytes;
-    static constexpr size_t smem = main_bytes + (NC + 1 + WARPS + 4) * sizeof(int);
+    static constexpr size_t main_bytes = field_bytes > rec_bytes || SHARED ? field_bytes : rec_bytes;
+    static constexpr size_t smem = main_bytes + (SHARED ? 8 * WSZ : NC + 1 + WARPS + 4) * sizeof(int);
 };
 
 template <typename S, typename FT, bool FIRST>
@@ -632,11 +656,13 @@ k_move_deposit(int64_t n_per_sort, int Ns, int N, int fineness, double h, double
     constexpr int CX = S::CX, NC = S::NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // the field window (FieldWin); after the gather, over it, the particles'
-    // records in the order of their cells
+    // records in the order of their cells (SHARED: behind it, the node sums)
     unsigned char *sf = smem_raw;
     double *rec = reinterpret_cast<double *>(smem_raw);
     int *start = reinterpret_cast<int *>(smem_raw + S::main_bytes);   // [NC + 1] first records
     int *wsum = start + NC + 1, *box = wsum + S::WARPS;
+    unsigned *sum_lo = reinterpret_cast<unsigned *>(smem_raw + S::main_bytes);   // SHARED: [4][WX][WY]
+    int *sum_hi = reinterpret_cast<int *>(sum_lo + 4 * WSZ);
     const int s = blockIdx.z;
     const int64_t base = (int64_t)s * n_per_sort;
     const int half_n = N / 2;
@@ -718,8 +744,8 @@ k_move_deposit(int64_t n_per_sort, int Ns, int N, int fineness, double h, double
     const int px = origin((max((int)blockIdx.y * S::TI - shift, 0) - mid) * lat);
     const int py = origin(((int)blockIdx.x * S::TJ - mid) * lat);
     fill(px, py);
-    for (int t = threadIdx.x; t <= NC; t += blockDim.x) start[t] = 0;
-    if (threadIdx.x < 4) box[threadIdx.x] = (threadIdx.x & 1) ? -1 : 0x7fffffff;
+    for (int t = threadIdx.x; t < (S::SHARED ? 8 * WSZ : NC + 1); t += blockDim.x) start[t] = 0;
+    if (!S::SHARED && threadIdx.x < 4) box[threadIdx.x] = (threadIdx.x & 1) ? -1 : 0x7fffffff;
     const int off = cell_of(r0x * ih + 0.5, half_n, dummy) != cell_of(r1x * ih + 0.5, half_n, dummy);
     if (off != shift) load(off);
     if ((int)blockIdx.y * S::TI - off >= Ns) return;
@@ -767,7 +793,6 @@ k_move_deposit(int64_t n_per_sort, int Ns, int N, int fineness, double h, double
         if (yh < -boundary) { yh = -2 * boundary - yh; z = true; }
         zero_p[p] = z;
         double xl, yl;
-        // FP64: the quotient of K2 itself; mixed: the reciprocal
         ix[p] = cell_of(xh * ih + 0.5, half_n, xl);
         iy[p] = cell_of(yh * ih + 0.5, half_n, yl);
         xlf[p] = (FT)xl; ylf[p] = (FT)yl;
@@ -984,6 +1009,76 @@ k_move_deposit(int64_t n_per_sort, int Ns, int N, int fineness, double h, double
     }
 
     // ---- phase 4: deposit ----
+    if constexpr (S::SHARED) {
+        // Two particles in the same or neighbouring cells share a footprint of
+        // 6 x 6 nodes, their terms added before the atomics (each still rounded
+        // by itself); any other pair goes one by one.
+        const int mx = min(cx[0], cx[1]), my = min(cy[0], cy[1]);
+        const int lx = mx - 2 - wx0, ly = my - 2 - wy0;
+        if (cx[0] >= 0 && cx[1] >= 0 && abs(cx[1] - cx[0]) <= 1 && abs(cy[1] - cy[0]) <= 1 && lx >= 0 &&
+            lx + 6 <= WX && ly >= 0 && ly + 6 <= WY && max_abs4(sv[0]) < FIX_SHARED_LIMIT &&
+            max_abs4(sv[1]) < FIX_SHARED_LIMIT) {
+            double ax[6], ay[6], bx[6], by[6], t[5];
+            weights4(dxl[0], t); shift6(t, cx[0] - mx, ax);
+            weights4(dyl[0], t); shift6(t, cy[0] - my, ay);
+            weights4(dxl[1], t); shift6(t, cx[1] - mx, bx);
+            weights4(dyl[1], t); shift6(t, cy[1] - my, by);
+            const bool wide = cy[0] != cy[1];
+            int row = lx * WY + ly;
+#pragma unroll 1
+            for (int a = 0; a < 6; a++) {
+#pragma unroll
+                for (int b = 0; b < 6; b++) {
+                    if (b == 5 && !wide) continue;
+                    const double wa = ax[0] * ay[b], wb = bx[0] * by[b];
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        shared_fix_add(sum_lo + q * WSZ + row + b, sum_hi + q * WSZ + row + b,
+                                       fma(sv[0][q], wa, fma(sv[1][q], wb, FIX_MAGIC)));
+                }
+#pragma unroll
+                for (int k = 0; k < 5; k++) { ax[k] = ax[k + 1]; bx[k] = bx[k + 1]; }
+                row += WY;
+            }
+        } else {
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                if (cx[p] < 0) continue;
+                const int px = cx[p] - 2 - wx0, py = cy[p] - 2 - wy0;
+                if (!(px >= 0 && px + 5 <= WX && py >= 0 && py + 5 <= WY && max_abs4(sv[p]) < FIX_SHARED_LIMIT)) {
+                    deposit_direct<FT>(g4, N, cx[p], cy[p], dxl[p], dyl[p], sv[p]);
+                    continue;
+                }
+                double wx[5], wy[5];
+                weights4(dxl[p], wx);
+                weights4(dyl[p], wy);
+                int row = px * WY + py;
+#pragma unroll 1
+                for (int a = 0; a < 5; a++) {
+#pragma unroll
+                    for (int b = 0; b < 5; b++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            shared_fix_add(sum_lo + q * WSZ + row + b, sum_hi + q * WSZ + row + b,
+                                           fma(sv[p][q], wx[0] * wy[b], FIX_MAGIC));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) wx[k] = wx[k + 1];
+                    row += WY;
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            for (int t = threadIdx.x; t < WSZ; t += THREADS) {
+                const unsigned lo = sum_lo[q * WSZ + t];
+                const int hi = sum_hi[q * WSZ + t];
+                if (lo || hi)
+                    atomicAdd(g4[q] + (int64_t)(wx0 + t / WY) * N + wy0 + t % WY,
+                              (Acc)(((long long)hi << 20) + lo));
+            }
+        return;
+    }
     // Particles whose stencil lies in the window are counted per cell; the
     // others (and, in mixed precision, values outside the window's range) go
     // straight to HBM.
@@ -1147,7 +1242,7 @@ static int dispatch_move_deposit(const lcb_move_deposit_args *a,
                                       typename StageAcc<FT>::type *const out[4], cudaStream_t st)
 {
     typedef Stage<FT, 20, 28> Two;
-    typedef Stage<FT, 28, 44> One;
+    typedef Stage<FT, 28, 44, sizeof(FT) == 4> One;
     if (a->lattice_fineness >= 2)
         return a->first ? launch_move_deposit<Two, FT, true>(a, out, st)
                         : launch_move_deposit<Two, FT, false>(a, out, st);
