@@ -814,15 +814,26 @@ NCU_TRAFFIC = {("move_deposit", "fp64"): 118.4e6}
 STAGE_BYTES = 664.0 / 3
 
 
+# 8-byte values per grid node and field solve by the fast transforms: four
+# currents of two planes each, full and previous (16), two beam densities and
+# the four fields of the Helmholtz terms; then, in the xi step's first solve,
+# two previous fields and six half-step outputs, in its second six previous
+# fields and seven outputs twice.  Mean of the two.
+SOLVE_VALUES = 22 + (8 + 20) / 2
+
+
 def op_roofline(name, o, N, Np, precision, peaks):
-    """Roofline of one op from its per-call CUDA-event time `o["ms_avg"]`:
-    compute_fields against the measured bf16 burst peak with the useful
-    dense-transform flops 56 N^3 per call (two calls per xi step make the
-    112 N^3 per xi step of the transforms as dense contractions), the fused
-    particle stage against the measured HBM copy bandwidth with 664 / 3 B
-    per particle (the xi step's 664 B over its three stages)."""
+    """Roofline of one op from its per-call CUDA-event time `o["ms_avg"]`,
+    against the measured HBM copy bandwidth: compute_fields with its inputs
+    and outputs once (its transforms, some 0.2 GFLOP of FP64 at N = 513, take
+    less), the fused particle stage with 664 / 3 B per particle (the xi step's
+    664 B over its three stages).  On grids without fast transforms
+    compute_fields goes against the measured bf16 burst peak with the useful
+    flops of its dense transforms, 56 N^3 per call."""
+    from lcodepy_b200 import _lib
     sec = o["ms_avg"] / 1e3
-    if name == "compute_fields":
+    prec = _lib.LCB_PREC_MIXED if precision == "mixed" else _lib.LCB_PREC_FP64
+    if name == "compute_fields" and _lib.load().lcb_wave_kernel_choice(N, prec) != 3:
         # without the measured peaks: 1.59 PFLOP/s, an earlier burst
         # measurement of cuBLAS bf16 on B200
         peak = peaks.get("bf16_tflops", 1590.0)
@@ -835,11 +846,14 @@ def op_roofline(name, o, N, Np, precision, peaks):
                 "peak_source": ("measured bf16 burst" if "bf16_tflops" in peaks
                                 else "fallback 1590 TFLOP/s")}
     peak = peaks.get("hbm_gbs", 6650.0)
-    nbytes = STAGE_BYTES * Np
+    if name == "compute_fields":
+        nbytes, work = SOLVE_VALUES * 8 * N * N, f"{SOLVE_VALUES:g} x 8 B x {N}^2 nodes"
+    else:
+        nbytes, work = STAGE_BYTES * Np, f"664/3 B x {Np} particles"
     achieved = nbytes / sec / 1e9
     return {"bound": "hbm", "kernel": name, "achieved": achieved, "peak": peak,
             "unit": "GB/s", "frac": achieved / peak,
-            "work_per_launch": f"{nbytes:.4g} B (664/3 B x {Np} particles)",
+            "work_per_launch": f"{nbytes:.4g} B ({work})",
             "traffic": NCU_TRAFFIC.get((name, precision)),
             "peak_source": "measured" if "hbm_gbs" in peaks else "fallback 6650 GB/s"}
 

@@ -38,3 +38,15 @@ def test_two_rank_max_over_ranks_and_barrier():
         out = m.dict()
         mp.spawn(_rank, args=(ws, port, out), nprocs=ws, join=True)
         assert dict(out) == {0: 2.5, 1: 2.5}
+
+
+def test_roofline_of_the_solver_that_runs():
+    """Grids with fast transforms are rated by their bytes, the others by the
+    flops of the dense products."""
+    import bench
+    peaks = {"hbm_gbs": 6000.0, "bf16_tflops": 1500.0}
+    for N, bound, work in ((513, "hbm", 36 * 8 * 513 ** 2 / 6000e9), (39, "tensor", 56 * 39 ** 3 / 1500e12)):
+        for precision in ("fp64", "mixed"):
+            r = bench.op_roofline("compute_fields", {"ms_avg": 1.0}, N, 1, precision, peaks)
+            assert r["bound"] == bound
+            assert abs(r["frac"] - work / 1e-3) < 1e-12
