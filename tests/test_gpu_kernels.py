@@ -324,8 +324,8 @@ def test_compute_fields(golden, precision, rel):
 @pytest.mark.parametrize("N", [33, 129, 257, 513])
 def test_compute_fields_sizes_vs_oracle(N, precision, rel):
     """Random currents at several grid sizes, up to the production grid 513
-    (every tiling of the tensor-core waves: 32- and 64-wide tiles, eight and
-    four slices, the stage counts of each grid)."""
+    (by the fast transforms; test_gpu_spectral.py takes the same sizes, and
+    grids without fast transforms, through the tensor-core waves)."""
     L = _lib.load()
     h, dxi = 0.05, 0.05
     rng = np.random.default_rng(N)

@@ -1,9 +1,10 @@
 """Field solves on either side of the choice between the fast transforms
 (N - 1 a product of primes up to 13) and the dense tensor-core products:
-every radix, the lengths with their own kernels and the smallest grids,
-against the oracle.  The fast transforms run in FP64 in both precisions, so
-both are held to the FP64 bound: two transforms and back of at most 2 N
-points with a spectral factor lose a few tens of 2^-53 of the field's
+every radix, the lengths with their own kernels, both kernels of the columns
+(two columns a block below 1,100 points a line, one above) and the smallest
+grids, against the oracle.  The fast transforms run in FP64 in both
+precisions, so both are held to the FP64 bound: two transforms and back of at
+most 2 N points with a spectral factor lose a few tens of 2^-53 of the field's
 largest value; the factor's spread (a condition of at most N^2) multiplies
 the right-hand side's own rounding, which both sides share."""
 import pytest
@@ -15,6 +16,9 @@ if not torch.cuda.is_available():  # pragma: no cover
     pytest.skip("needs CUDA", allow_module_level=True)
 
 import ctypes as C  # noqa: E402
+import os  # noqa: E402
+import subprocess  # noqa: E402
+import sys  # noqa: E402
 
 import numpy as np  # noqa: E402
 
@@ -28,18 +32,34 @@ BOTH = (_lib.LCB_PREC_FP64, _lib.LCB_PREC_MIXED)
 
 
 @pytest.mark.parametrize("precision", BOTH)
-@pytest.mark.parametrize("N", [9, 11, 15, 19, 23, 27, 51, 65, 79, 91, 111, 155, 193, 321, 331, 385])
+@pytest.mark.parametrize("N", [9, 11, 15, 19, 23, 27, 51, 55, 65, 79, 91, 111, 133, 155, 193, 321, 331, 385, 551, 577, 641])
 def test_fast_transforms_vs_oracle(N, precision):
     check(N, precision, 1e-11)
     assert _lib.load().lcb_wave_kernel_choice(N, precision) == 3
 
 
 @pytest.mark.parametrize("precision,rel", [(_lib.LCB_PREC_FP64, 1e-11), (_lib.LCB_PREC_MIXED, 3e-5)])
-@pytest.mark.parametrize("N", [39, 95, 259])
+@pytest.mark.parametrize("N", [35, 39, 95, 139, 259, 495, 519])
 def test_dense_transforms_vs_oracle(N, precision, rel):
-    """Grids with a larger prime factor in N - 1 (19, 47, 43)."""
+    """Grids with a larger prime factor in N - 1 (17, 19, 47, 23, 43, 19, 37):
+    32- and 64-wide tiles, eight and four slices, full and ragged ones."""
     check(N, precision, rel)
     assert _lib.load().lcb_wave_kernel_choice(N, precision) in (1, 2)
+
+
+@pytest.mark.parametrize("kernel", ["tiled", "persistent"])
+def test_either_wave_kernel_on_grids_with_fast_transforms(kernel):
+    """LCB_WAVE_KERNEL, read once per process, takes the dense products for
+    every grid."""
+    code = ("import sys; sys.path[:0] = sys.argv[1:]\n"
+            "from test_gpu_kernels import _lib, test_compute_fields_sizes_vs_oracle as check\n"
+            "for N in (33, 129, 257, 513):\n"
+            "    check(N, _lib.LCB_PREC_FP64, 1e-11)\n"
+            "    check(N, _lib.LCB_PREC_MIXED, 3e-5)\n"
+            "    assert _lib.load().lcb_wave_kernel_choice(N, _lib.LCB_PREC_FP64) != 3\n")
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.run([sys.executable, "-c", code, os.path.dirname(here), here], check=True, timeout=300,
+                   env={**os.environ, "LCB_WAVE_KERNEL": kernel})
 
 
 @pytest.mark.parametrize("small", ["transverse currents", "charge"])

@@ -129,3 +129,68 @@ def test_background_cancels_the_electrons_at_rest(N, ppc):
     np.testing.assert_array_equal(out.buf[0][1].cpu().numpy(), ps.ro_initial.cpu().numpy())
     assert abs(left.mean()) <= 4 * 1.5 * 2.0 ** -53 / left.size ** 0.5
     assert (left ** 2).mean() ** 0.5 <= 2.5 * 2.0 ** -53
+
+
+def _compare_with_separate(ps, rel):
+    prev, full = ps.states
+    F = ps.fields[0]
+    start = {k: getattr(full, k).clone() for k in NAMES}
+    ps._move_smart(F, prev, full)
+    want, out = CurrentSet(ps.N, DEV), CurrentSet(ps.N, DEV)
+    ps._deposit(full, want)
+    for k, v in start.items():
+        getattr(full, k).copy_(v)
+    ps._move_deposit(F, prev, full, out, False)
+    torch.cuda.synchronize()
+    assert int(ps.err.item()) == 0
+    for i, k in enumerate(("ro", "jx", "jy", "jz")):
+        _close(out.buf[i], want.buf[i], rel, k)
+    return want.buf[0][0]
+
+
+@pytest.mark.parametrize("precision,rel", [("fp64", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("ppc,share", [(1, 0.98), (4, 0.98), (4, 0.7), (9, 0.98)])
+def test_stage_where_a_tile_meets_in_few_cells(ppc, share, precision, rel):
+    """A density spike: the particles of every 16 x 32 of the lattice drawn
+    together to a point, so that one cell holds hundreds."""
+    ps = _solver(97, ppc, "background", precision)
+    prev, full = ps.states
+    Ns = prev.Ns
+    i = torch.arange(Ns, device=DEV)
+    for k, tile in (("x", 16), ("y", 32)):
+        at = getattr(prev, k + "_init").view(Ns, Ns)
+        u = at[:, 0] if k == "x" else at[0]
+        to = u[(i // tile * tile + tile // 2).clamp(max=Ns - 1)]
+        d = (to - u) * share
+        for s in (prev, full):
+            getattr(s, k + "_offt").copy_((d[:, None] if k == "x" else d[None]).expand(Ns, Ns).reshape(-1))
+    for s in (prev, full):
+        for k in ("px", "py", "pz"):
+            getattr(s, k).mul_(0.1)
+    # (512 particles of 1 / ppc each in a cell, weights up to 0.6^2)
+    assert float(_compare_with_separate(ps, rel).abs().max()) > (0.5 * 512 / ppc * 0.36 if share > 0.9 else 3)
+
+
+@pytest.mark.parametrize("ppc", [1, 4])
+@pytest.mark.parametrize("precision,big,rel", [("fp64", 1e201, 1e-12), ("fp64", 1e199, 1e-12), ("mixed", 4096.0, 1e-8)])
+def test_stage_with_values_out_of_a_blocks_range(ppc, precision, big, rel):
+    """Particles whose density reaches what a block does not sum (FP64 1e200,
+    mixed 2^10) go to HBM by themselves; the others stay as they are."""
+    ps = _solver(65, ppc, "background", precision)
+    prev, full = ps.states
+    n = prev.n_per_sort
+    ps.fields[0].buf.zero_()
+    k = n // 2 + 11
+    for s in (prev, full):
+        s.q[k] = big * ps.h ** 2
+        s.x_offt[k] = s.y_offt[k] = s.px[k] = s.py[k] = s.pz[k] = 0
+    top = _compare_with_separate(ps, rel)
+    assert 0.1 * big < float(top.abs().max()) < big
+    far = torch.ones(ps.N, ps.N, dtype=torch.bool, device=DEV)
+    at = int(top.abs().argmax())
+    far[at // ps.N - 5:at // ps.N + 6, at % ps.N - 5:at % ps.N + 6] = False
+    got, want = CurrentSet(ps.N, DEV), CurrentSet(ps.N, DEV)
+    ps._deposit(full, want)
+    ps._move_deposit(ps.fields[0], prev, full, got, False)
+    for a, b in zip(got.buf, want.buf):
+        _close(a[0][far], b[0][far], 1e-12 if precision == "fp64" else 1e-5, "elsewhere")
