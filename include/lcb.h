@@ -42,7 +42,8 @@ extern "C" {
 
 /* Precision modes for the field solver and deposition. */
 #define LCB_PREC_FP64 0   /* FP64 everywhere: the reference's arithmetic */
-#define LCB_PREC_MIXED 1  /* fixed-point deposition, FP32 transforms; FP64 particles */
+#define LCB_PREC_MIXED 1  /* fixed-point deposition, FP32 gather; FP64 particles; FP32-accurate
+                             fields on grids without fast transforms, else FP64 */
 
 const char *lcb_last_error(void);
 int lcb_version(void);
@@ -177,16 +178,19 @@ typedef struct lcb_compute_fields_args {
 
 /* Replaces compute_fields, lcode/plasma3d/fields.py:276-322 (with
  * calculate_Ex_Ey_Bx_By :176-230, calculate_Ez :112-139, calculate_Bz
- * :233-266, calculate_Phi :142-159 and the GPU transforms :36-107): every
- * DST-I / DCT-I / mixed transform is a dense batched matrix product.
- * Phi is skipped when both its out_full and out_half planes are NULL.
- * The transforms run on one of two tensor-core wave kernels (one CTA per
- * output tile, or a persistent warp-specialised one); the first call for a
- * (device, grid_steps, precision) that is not under stream capture times
- * both on the caller's stream and keeps the faster (it computes the same
- * outputs several times and synchronises the stream once).
- * LCB_WAVE_KERNEL=tiled or =persistent in the environment fixes the choice,
- * for every grid. */
+ * :233-266, calculate_Phi :142-159 and the GPU transforms :36-107).  Phi is
+ * skipped when both its out_full and out_half planes are NULL.
+ * Grids whose N - 1 has prime factors up to 13 only and at most 3124 intervals
+ * (every smaller grid that the configuration gives) are solved by fast
+ * transforms, FP64 in both precisions; nothing is timed or synchronised.
+ * On the others every DST-I / DCT-I / mixed transform is a dense batched
+ * matrix product, FP64- or FP32-accurate, on one of two tensor-core wave
+ * kernels (one CTA per output tile, or a persistent warp-specialised one): the
+ * first call for a (device, grid_steps, precision) that is not under stream
+ * capture times both on the caller's stream and keeps the faster (it computes
+ * the same outputs several times and synchronises the stream once).
+ * LCB_WAVE_KERNEL=tiled or =persistent in the environment takes the dense
+ * products, and that kernel, for every grid. */
 int lcb_compute_fields(const lcb_compute_fields_args *a, void *stream);
 size_t lcb_compute_fields_workspace_bytes(int grid_steps, int precision);
 

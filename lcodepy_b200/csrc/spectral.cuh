@@ -1,5 +1,6 @@
 // Field solver by fast transforms, for grids whose number of intervals N - 1
-// factors into small primes (every grid the configuration gives).
+// factors into small primes, as the configuration's do, up to 3125 nodes a side
+// (two buffers of a line in a block's shared memory).
 #pragma once
 
 #include "common.cuh"
