@@ -44,8 +44,8 @@
 // (four launches instead of eleven), at 331, with the kernels for any length,
 // from 84 to 52 us.  Finding the scales costs 0.5 to 1.5 us of each kernel of
 // the rows and of the right-hand sides; without them (one rounding size for all
-// the fields of a unit) 385 takes 48.0 us instead of 49.5, 641 139 instead of
-// 141.  The error against 64-bit sums is 6e-16 of each field (dense: 1e-14
+// the fields of a unit) 385 takes 48.3 us instead of 48.9, 451 80.2 instead of
+// 81.0, 641 138.6 instead of 141.  The error against 64-bit sums is 6e-16 of each field (dense: 1e-14
 // FP64, 1e-6 mixed, at 513).
 #include <map>
 #include <mutex>
@@ -632,13 +632,27 @@ k_rows_any(int N, const __grid_constant__ DftPlan p, const double2 *tw, double2 
     double2 *row = Z + ((int64_t)unit * N + i) * 2 * pitch;
     double2 *a = line, *b = line + sp_line(L);
     if (DIR == 0) {
+        // four nodes of a thread on their way at a time, the first ones while
+        // the scales are found (451: 83.0 us without, 81.0 with)
+        double2 A[4], B[4];
         double f[4];
-        sp_scales<SP_ANY_THREADS>(sc, unit, blocks, phi_shift, i == 0, red2, f);
-        for (int idx = threadIdx.x; idx <= M; idx += SP_ANY_THREADS) {
-            double2 zp, zm;
-            sp_pack(row[idx], row[pitch + idx], f, zp, zm);
-            a[sp_pad(idx)] = zp;
-            if (idx > 0 && idx < M) a[sp_pad(L - idx)] = zm;
+        for (int r = 0; r <= M; r += 4 * SP_ANY_THREADS) {
+            const int j0 = r + threadIdx.x;
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                const int j = j0 + g * SP_ANY_THREADS;
+                if (j <= M) { A[g] = row[j]; B[g] = row[pitch + j]; }
+            }
+            if (r == 0) sp_scales<SP_ANY_THREADS>(sc, unit, blocks, phi_shift, i == 0, red2, f);
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                const int j = j0 + g * SP_ANY_THREADS;
+                if (j > M) continue;
+                double2 zp, zm;
+                sp_pack(A[g], B[g], f, zp, zm);
+                a[sp_pad(j)] = zp;
+                if (j > 0 && j < M) a[sp_pad(L - j)] = zm;
+            }
         }
     } else {
         for (int idx = threadIdx.x; idx < L; idx += SP_ANY_THREADS)
