@@ -55,7 +55,7 @@ default_config_values = {
 # Extra keys understood by this package only (the reference ignores unknown
 # keys, so adding them keeps configs interchangeable).
 #   'precision': 'fp64' (default; the reference's arithmetic) or 'mixed'
-#                (FP32 deposition and FP32 transforms, FP64 particles).
+#                (fixed-point deposition, FP32 gather, FP64 particles).
 #   'deposit-precision', 'field-precision': 'fp64' or 'fp32', overriding
 #                'precision' for the deposition or the field solve alone.
 #   'print-every': xi steps between the on-axis Ez lines (reference: 10).

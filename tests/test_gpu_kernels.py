@@ -2,8 +2,8 @@
 oracle and the reference's own known answers (tests/golden/kat_*.npz).
 
 Tolerances: the kernels compute in FP64 like the reference; the GPU sums in
-a different order (atomics, fused multiply-adds, dense transforms instead of
-FFTs), so results agree to a few ulps of the largest element."""
+a different order (atomics, fused multiply-adds, transforms of packed or dense
+lines), so results agree to a few ulps of the largest element."""
 import ctypes as C
 
 import numpy as np

@@ -164,7 +164,7 @@ def test_two_time_steps_beam_push_vs_oracle():
 
 
 def test_mixed_precision_on_axis_ez():
-    """FP32 deposition and FP32 transforms, FP64 particles: on-axis Ez within
+    """Fixed-point deposition and FP32 gather, FP64 particles: on-axis Ez within
     relative L2 1e-5 of the FP64 run (rigid driver, 129 x 129, 201 xi steps)."""
     base = cfg(**{'rigid-beam': True, 'window-width': 6.5, 'transverse-step': 0.1,
                   'xi-step': 0.1, 'window-length': 20})
